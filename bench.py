@@ -219,7 +219,7 @@ def run_ours(args):
     value = job_rate(n_moving * steps_total, world, max_ms)
 
     # roofline of the dominant kernel: one time step's force evaluation and
-    # integration (k_detect + k_contacts + k_sum), timed with CUDA events on
+    # integration (k_units + k_sum), timed with CUDA events on
     # the engine's stream at the state where the timed window ended
     fk_ms = eng.time_force_kernel(20)
     cnt = eng.counts()
@@ -277,7 +277,7 @@ def run_ours(args):
                 "step": f"upload + initial evaluation + {window} time steps + download, {e2e_runs} runs"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic,
-                     "kernel": "one time step's force evaluation + integration: k_detect + k_contacts + k_sum",
+                     "kernel": "one time step's force evaluation + integration: k_units + k_sum",
                      "peak_source": peak_kind, "bytes_per_launch": fk_bytes, "launch_ms": fk_ms,
                      "bytes_model": "N x 248 B + C x B_c (B_c = 160 B with rolling and torsion springs)"},
         "cpu_baseline": cpu,

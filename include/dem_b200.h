@@ -350,8 +350,9 @@ typedef struct dem_cg_grid {
  * how the work is spread over the GPU, never the arithmetic: results are
  * bit-identical under every shape. */
 typedef struct dem_tuning {
-    int32_t detect_block;            /* threads per block of the contact predicate: 64, 128 or 256 */
-    int32_t contacts_blocks_per_sm;  /* resident blocks (of 128) per SM of the contact-law kernel,
+    int32_t detect_block;            /* pairs and walls a block of the contact kernel takes at a
+                                        time, in fours: 64, 128 or 256 (256, 512 or 1024 of them) */
+    int32_t contacts_blocks_per_sm;  /* resident blocks (of 128) per SM of the contact kernel,
                                         3..6, with the register budget they leave (168 .. 85) */
     int32_t sum_block;               /* threads per block of the sum/integration kernel: 64, 128, 256 */
     int32_t reserved;

@@ -93,7 +93,7 @@ struct Handle {
     int rb_grid = 148;                 // blocks of the cooperative rebuild (all resident)
     std::vector<int> level_buf;        // HGrid level of every particle (one-instance uploads)
     // launch shapes of the force kernels (dem_autotune / dem_set_tuning)
-    dem_tuning tune{DETECT_BLOCK, 4, SUM_BLOCK, 0, 0.0, 0.0};
+    dem_tuning tune{DETECT_TUNE, 4, SUM_BLOCK, 0, 0.0, 0.0};
     // optional events between the force kernels, for the autotuner's
     // per-kernel times (null outside a measurement)
     cudaEvent_t* kev = nullptr;
@@ -188,51 +188,44 @@ void launch_insert(Handle* h, cudaStream_t s)
     if (h->n_ins_launch > 0)
         k_insert<<<h->n_ins_inst, INS_THREADS, 0, s>>>(h->d, ins_ptrs(h));
 }
-constexpr int FORCE_LAUNCHES = 3;
+constexpr int FORCE_LAUNCHES = 2;
 
 // Law variants the force kernel is instantiated for; the handle uses a
 // specialised one when every species pair shares the same law pair.
 enum LawVariant { LAW_GENERIC = 0, LAW_LINEAR_SLIDING, LAW_LINEAR_ROLLING, LAW_HERTZ_MINDLIN, LAW_HERTZ_MINDLIN_RT };
 
-// one force evaluation: detect -> contacts -> sum (+ integration for MODE 1);
-// RECORD: the evaluation may be the last of the call (contact records)
+// one force evaluation: units -> sum (+ integration for MODE 1); RECORD: the
+// evaluation may be the last of the call (contact records)
 template <int MODE, int NLAW, int FLAW, int NCOMP, bool RECORD>
 void launch_pipeline(Handle* h, cudaStream_t s)
 {
     DevPtrs& d = h->d;
     if (h->kev) cudaEventRecord(h->kev[0], s);
-    switch (h->tune.detect_block) {
-    case 64: k_detect<MODE, NCOMP, 64><<<grid_for(d.n, 64), 64, 0, s>>>(d); break;
-    case 256: k_detect<MODE, NCOMP, 256><<<grid_for(d.n, 256), 256, 0, s>>>(d); break;
-    default: k_detect<MODE, NCOMP, DETECT_BLOCK><<<grid_for(d.n, DETECT_BLOCK), DETECT_BLOCK, 0, s>>>(d);
-    }
-    if (h->kev) cudaEventRecord(h->kev[1], s);
-    // one resident wave of tune.contacts_blocks_per_sm blocks of 128 per SM,
-    // grid-stride over the items; the time-step variant without records is
-    // compiled with that many blocks' register budget (3 to 6), the others
-    // with 4 (128 registers)
+    // one resident wave of tune.contacts_blocks_per_sm blocks of 128 per SM over
+    // the units; the time-step variant without records is compiled with that
+    // many blocks' register budget (3 to 6), the others with 4 (128 registers)
     const int bpsm = (MODE == 1 && !RECORD) ? h->tune.contacts_blocks_per_sm : 4;
-    const unsigned gc = (unsigned)std::max(1, std::min((d.item_cap + CONTACT_BLOCK - 1) / CONTACT_BLOCK,
-                                                       h->sm_count * bpsm));
+    const unsigned gc = (unsigned)std::max(1, std::min((d.unit_cap + 31) / 32, h->sm_count * bpsm));
+    const int chunk = UNIT_CHUNK_PER_TUNE * h->tune.detect_block;
     if (MODE == 1 && !RECORD && bpsm == 3)
-        k_contacts<MODE, NLAW, FLAW, NCOMP, RECORD, 3><<<gc, CONTACT_BLOCK, 0, s>>>(d);
+        k_units<MODE, NLAW, FLAW, NCOMP, RECORD, 3><<<gc, UNIT_BLOCK, 0, s>>>(d, chunk);
     else if (MODE == 1 && !RECORD && bpsm == 5)
-        k_contacts<MODE, NLAW, FLAW, NCOMP, RECORD, 5><<<gc, CONTACT_BLOCK, 0, s>>>(d);
+        k_units<MODE, NLAW, FLAW, NCOMP, RECORD, 5><<<gc, UNIT_BLOCK, 0, s>>>(d, chunk);
     else if (MODE == 1 && !RECORD && bpsm == 6)
-        k_contacts<MODE, NLAW, FLAW, NCOMP, RECORD, 6><<<gc, CONTACT_BLOCK, 0, s>>>(d);
+        k_units<MODE, NLAW, FLAW, NCOMP, RECORD, 6><<<gc, UNIT_BLOCK, 0, s>>>(d, chunk);
     else
-        k_contacts<MODE, NLAW, FLAW, NCOMP, RECORD, 4><<<gc, CONTACT_BLOCK, 0, s>>>(d);
+        k_units<MODE, NLAW, FLAW, NCOMP, RECORD, 4><<<gc, UNIT_BLOCK, 0, s>>>(d, chunk);
     if (d.has_tri) { // at most one triangle item per particle
         const unsigned gt = (unsigned)std::max(1, std::min((d.n + TRI_BLOCK - 1) / TRI_BLOCK, h->sm_count * 4));
         k_tri<MODE, NLAW, FLAW, NCOMP><<<gt, TRI_BLOCK, 0, s>>>(d);
     }
-    if (h->kev) cudaEventRecord(h->kev[2], s);
+    if (h->kev) cudaEventRecord(h->kev[1], s);
     switch (h->tune.sum_block) {
     case 64: k_sum<MODE, 64><<<grid_for(d.n, 64), 64, 0, s>>>(d); break;
     case 256: k_sum<MODE, 256><<<grid_for(d.n, 256), 256, 0, s>>>(d); break;
     default: k_sum<MODE, SUM_BLOCK><<<grid_for(d.n, SUM_BLOCK), SUM_BLOCK, 0, s>>>(d);
     }
-    if (h->kev) cudaEventRecord(h->kev[3], s);
+    if (h->kev) cudaEventRecord(h->kev[2], s);
 }
 int force_launches(const Handle* h) { return FORCE_LAUNCHES + (h->d.has_tri ? 1 : 0); }
 
@@ -1040,6 +1033,9 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
         std::min<long long>(2000000000ll, h->cfg.max_contacts > 0
                                               ? (long long)n * h->cfg.max_contacts + 1024
                                               : (long long)n * std::min(cap, 16) + (long long)n * std::min(wmax, 4) + 1024);
+    // units: a pair is in both particles' rows, so at most cap / 2 pairs per
+    // particle, plus its walls (all triangles are one unit)
+    const long long unit_cap = std::min<long long>(2147000000ll, (long long)n * (cap / 2 + std::min(wmax, 32) + 1) + 32);
     // ---- (re)allocate: a re-upload with the same sizes keeps the device arrays
     // and the captured graphs (their kernel arguments stay valid)
     const unsigned record_capacity = (unsigned)std::min<long long>(
@@ -1070,6 +1066,9 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
     d.n_species_table = (int)h->species.size();
     d.zero_idist = 1;
     for (const auto& sp : h->species) d.zero_idist = d.zero_idist && sp.interaction_distance == 0.0;
+    d.any_periodic = 0;
+    for (const auto& in : h->inst_desc) d.any_periodic = d.any_periodic || (in.periodic_mask & 7u);
+    d.unit_cap = (int)unit_cap;
     d.has_tri = 0;
     for (const auto& w : h->walls) d.has_tri = d.has_tri || w.type == DEM_WALL_TRIANGLE;
     d.dt = h->cfg.time_step;
@@ -1082,32 +1081,31 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
                           d.ncomp == kept.ncomp && d.wmax == kept.wmax && d.ncells == kept.ncells &&
                           d.rotation == kept.rotation && d.single_instance == kept.single_instance &&
                           d.n_species_table == kept.n_species_table && d.zero_idist == kept.zero_idist &&
-                          d.dt == kept.dt && d.drag == kept.drag && d.has_tri == kept.has_tri;
+                          d.dt == kept.dt && d.drag == kept.drag && d.has_tri == kept.has_tri &&
+                          d.any_periodic == kept.any_periodic;
         if (!same) free_graphs(h);
         for (int b = 0; b < 2; ++b) {
             d.pr[b] = kept.pr[b]; d.vm[b] = kept.vm[b]; d.wi[b] = kept.wi[b]; d.qo[b] = kept.qo[b];
-            d.info[b] = kept.info[b]; d.caller[b] = kept.caller[b]; d.nbr[b] = kept.nbr[b]; d.cnt[b] = kept.cnt[b];
-            d.own[b] = kept.own[b];
-            d.wcand[b] = kept.wcand[b];
-            d.pool[b] = kept.pool[b]; d.hidx[b] = kept.hidx[b];
-            d.act[b] = kept.act[b]; d.whist[b] = kept.whist[b]; d.wact[b] = kept.wact[b];
+            d.info[b] = kept.info[b]; d.caller[b] = kept.caller[b];
+            d.unit[b] = kept.unit[b]; d.uidx[b] = kept.uidx[b];
+            d.pool[b] = kept.pool[b]; d.whist[b] = kept.whist[b]; d.wact[b] = kept.wact[b];
         }
+        d.cnt = kept.cnt; d.own = kept.own; d.wcand = kept.wcand; d.ubase = kept.ubase; d.wbase = kept.wbase;
+        d.epair = kept.epair;
         d.force = kept.force; d.torque = kept.torque; d.key = kept.key; d.perm = kept.perm; d.newidx = kept.newidx;
         d.cell_count = kept.cell_count; d.cell_start = kept.cell_start; d.cell_cursor = kept.cell_cursor;
         d.block_sums = kept.block_sums; d.rb_barrier = kept.rb_barrier; d.inst = kept.inst; d.species = kept.species; d.walls = kept.walls;
         d.wgeom = kept.wgeom; d.n_walls = kept.n_walls; d.ctl = kept.ctl; d.records = kept.records;
         d.n_instances = kept.n_instances;
         d.pf = kept.pf; d.rows = kept.rows; d.row_slot = kept.row_slot;
-        d.rev = kept.rev; d.slot = kept.slot; d.slotw = kept.slotw; d.items = kept.items; d.shares = kept.shares;
+        d.shares = kept.shares;
         d.item_cap = kept.item_cap;
         d.tri_list = kept.tri_list;
         d.slott = kept.slott;
         d.tri_first = kept.tri_first;
         d.tri_first_n = kept.tri_first_n;
         for (int b = 0; b < 2; ++b) { // no history carries over from the previous simulation
-            CU(cudaMemsetAsync(d.cnt[b], 0, NC * sizeof(int), h->stream));
-            CU(cudaMemsetAsync(d.act[b], 0, (size_t)d.nwords * NC * sizeof(unsigned), h->stream));
-            CU(cudaMemsetAsync(d.wact[b], 0, NC * sizeof(unsigned), h->stream));
+            CU(cudaMemsetAsync(d.wact[b], 0, NC * sizeof(unsigned), h->stream)); // (the new control has no units)
         }
     } else {
     for (int b = 0; b < 2; ++b) {
@@ -1117,17 +1115,18 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
         if ((rc = dalloc(h, &d.qo[b], NC))) return rc;
         if ((rc = dalloc(h, &d.info[b], NC))) return rc;
         if ((rc = dalloc(h, &d.caller[b], NC))) return rc;
-        if ((rc = dalloc(h, &d.nbr[b], (size_t)cap * NC))) return rc;
-        if ((rc = dalloc(h, &d.cnt[b], NC))) return rc;
-        if ((rc = dalloc(h, &d.own[b], (size_t)d.nwords * NC))) return rc;
-        if ((rc = dalloc(h, &d.wcand[b], NC))) return rc;
+        if ((rc = dalloc(h, &d.unit[b], (size_t)unit_cap))) return rc;
+        if ((rc = dalloc(h, &d.uidx[b], (size_t)unit_cap))) return rc;
         if ((rc = dalloc(h, &d.pool[b], (size_t)hist_stride(d.ncomp) * item_cap))) return rc;
-        if ((rc = dalloc(h, &d.hidx[b], (size_t)cap * NC))) return rc;
-        if ((rc = dalloc(h, &d.act[b], (size_t)d.nwords * NC))) return rc;
-        if ((rc = dalloc(h, &d.whist[b], (size_t)hist_stride(d.ncomp) * wmax * NC))) return rc;
+        if ((rc = dalloc(h, &d.whist[b], any_tri ? (size_t)hist_stride(d.ncomp) * wmax * NC : 1))) return rc;
         if ((rc = dalloc(h, &d.wact[b], NC))) return rc;
     }
-    if ((rc = dalloc(h, &d.rev, (size_t)cap * NC))) return rc;
+    if ((rc = dalloc(h, &d.cnt, NC))) return rc;
+    if ((rc = dalloc(h, &d.own, (size_t)d.nwords * NC))) return rc;
+    if ((rc = dalloc(h, &d.wcand, NC))) return rc;
+    if ((rc = dalloc(h, &d.ubase, NC))) return rc;
+    if ((rc = dalloc(h, &d.wbase, NC))) return rc;
+    if ((rc = dalloc(h, &d.epair, (size_t)cap * NC))) return rc;
     if ((rc = dalloc(h, &d.rows, (size_t)cap * NC))) return rc;
     if ((rc = dalloc(h, &d.pf, NC))) return rc;
     if (any_free) {
@@ -1137,10 +1136,7 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
         if ((rc = dalloc(h, &h->d_ins_rows, NC))) return rc;
         if ((rc = dalloc(h, &h->d_ovf, (size_t)ncells + 1 + 2 * NC))) return rc;
     }
-    if ((rc = dalloc(h, &d.slot, (size_t)cap * NC))) return rc;
-    if ((rc = dalloc(h, &d.slotw, (size_t)wmax * NC))) return rc;
     d.item_cap = (int)item_cap;
-    if ((rc = dalloc(h, &d.items, (size_t)d.item_cap))) return rc;
     if ((rc = dalloc(h, &d.shares, (size_t)d.item_cap * SHARE))) return rc;
     if ((rc = dalloc(h, &d.tri_list, NC))) return rc;
     if ((rc = dalloc(h, &d.slott, NC))) return rc;
@@ -1360,30 +1356,31 @@ int dem_upload_contacts(dem_handle* hh, const dem_contacts_soa* cs)
     Control c;
     if ((rc = read_control(h, &c))) return rc;
     DevPtrs& d = h->d;
-    const int n = d.n, cur = c.cur, l = c.lbuf;
+    const int n = d.n, cur = c.cur, l = c.lbuf, hb = c.hcur, nu = c.n_units;
     const size_t NC = d.ncap;
+    const bool tri = d.has_tri != 0;
     std::vector<int4> info(n);
-    std::vector<double4> pr(n);
-    std::vector<int> cnt(n), nbr((size_t)d.cap * NC);
-    std::vector<unsigned> act((size_t)d.nwords * NC), wact(NC);
-    std::vector<int> hidx((size_t)d.cap * NC, 0);
-    std::vector<double> pool, whist((size_t)hist_stride(d.ncomp) * d.wmax * NC);
+    std::vector<int2> unit(nu);
+    std::vector<int> uidx(nu);
+    std::vector<unsigned> wact(NC), wcand(NC);
+    std::vector<double> pool, whist(tri ? (size_t)hist_stride(d.ncomp) * d.wmax * NC : 0);
     CU(cudaMemcpyAsync(info.data(), d.info[cur], n * sizeof(int4), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaMemcpyAsync(pr.data(), d.pr[cur], n * sizeof(double4), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaMemcpyAsync(cnt.data(), d.cnt[l], n * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaMemcpyAsync(nbr.data(), d.nbr[l], nbr.size() * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaMemcpyAsync(act.data(), d.act[cur], act.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaMemcpyAsync(wact.data(), d.wact[cur], wact.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaMemcpyAsync(whist.data(), d.whist[cur], whist.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaMemcpyAsync(hidx.data(), d.hidx[cur], hidx.size() * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaMemcpyAsync(unit.data(), d.unit[l], nu * sizeof(int2), cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaMemcpyAsync(uidx.data(), d.uidx[hb], nu * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaMemcpyAsync(wact.data(), d.wact[hb], wact.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaMemcpyAsync(wcand.data(), d.wcand, wcand.size() * sizeof(unsigned), cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaMemcpyAsync(whist.data(), d.whist[hb], whist.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
     CU(cudaStreamSynchronize(h->stream));
     // springs injected by an earlier call stay where they are in the pool
     const int stride = hist_stride(d.ncomp);
     long long used = 0;
-    for (int s = 0; s < n; ++s)
-        for (int k = 0; k < std::min(cnt[s], d.cap); ++k)
-            if ((act[(size_t)(k >> 5) * NC + s] >> (k & 31)) & 1u)
-                used = std::max<long long>(used, (long long)hidx[nbr_at(d.ncap, s, k)] + 1);
+    std::vector<std::pair<long long, int>> units(nu); // (P slot, I slot or wall) -> unit
+    auto unit_key = [](int s, int t) { return ((long long)s << 32) | (long long)(unsigned)t; };
+    for (int u = 0; u < nu; ++u) {
+        units[u] = {unit_key(unit[u].x, unit[u].y), u};
+        if (unit[u].y != UNIT_TRI) used = std::max<long long>(used, (long long)uidx[u] + 1);
+    }
+    std::sort(units.begin(), units.end());
     pool.resize((size_t)used * stride);
     if (used) {
         CU(cudaMemcpyAsync(pool.data(), d.pool[c.pcur], pool.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -1397,20 +1394,18 @@ int dem_upload_contacts(dem_handle* hh, const dem_contacts_soa* cs)
         auto it = std::lower_bound(ids.begin(), ids.end(), std::make_pair(id, -1));
         return (it != ids.end() && it->first == id) ? it->second : -1;
     };
-    // an entry with a new spring gets the next record of the pool
-    auto set_entry = [&](int s, int t, const double* spr, double sign) -> bool {
-        for (int k = 0; k < cnt[s]; ++k) {
-            if (nbr[nbr_at(d.ncap, s, k)] != t) continue;
-            const size_t e = nbr_at(d.ncap, s, k);
-            if (!((act[(size_t)(k >> 5) * NC + s] >> (k & 31)) & 1u)) {
-                hidx[e] = (int)(pool.size() / stride);
-                pool.resize(pool.size() + stride, 0.0);
-            }
-            for (int comp = 0; comp < d.ncomp; ++comp) pool[(size_t)hidx[e] * stride + comp] = sign * spr[comp];
-            act[(size_t)(k >> 5) * NC + s] |= 1u << (k & 31);
-            return true;
+    // a unit with a new spring gets the next record of the pool
+    auto set_unit = [&](int s, int t, const double* spr, double sign) -> bool {
+        const long long key = unit_key(s, t);
+        auto it = std::lower_bound(units.begin(), units.end(), std::make_pair(key, -1));
+        if (it == units.end() || it->first != key) return false;
+        int& q = uidx[it->second];
+        if (q < 0) {
+            q = (int)(pool.size() / stride);
+            pool.resize(pool.size() + stride, 0.0);
         }
-        return false;
+        for (int comp = 0; comp < d.ncomp; ++comp) pool[(size_t)q * stride + comp] = sign * spr[comp];
+        return true;
     };
     for (long long r = 0; r < cs->n; ++r) {
         const double* spr = cs->springs ? cs->springs + 9 * r : nullptr;
@@ -1425,27 +1420,31 @@ int dem_upload_contacts(dem_handle* hh, const dem_contacts_soa* cs)
             const int w = h->wall_grouped[wc] - h->inst[in].wall_begin;
             if (w < 0 || w >= h->inst[in].wall_end - h->inst[in].wall_begin)
                 return fail(h, DEM_ERR_BAD_INPUT, "contact refers to a wall outside the particle's instance");
-            for (int comp = 0; comp < d.ncomp; ++comp) whist[whist_at(d.ncap, d.ncomp, sp, w) + comp] = spr[comp];
-            wact[sp] |= 1u << w;
+            // a wall out of reach has no unit: its contact ends at the first evaluation
+            if (!((h->inst[in].tri_mask >> w) & 1u)) {
+                set_unit(sp, ~w, spr, 1.0);
+            } else if ((wcand[sp] >> w) & 1u) {
+                for (int comp = 0; comp < d.ncomp; ++comp) whist[whist_at(d.ncap, d.ncomp, sp, w) + comp] = spr[comp];
+                wact[sp] |= 1u << w;
+            }
             continue;
         }
         const int si = slot_of(cs->id_i[r]);
         if (si < 0) return fail(h, DEM_ERR_BAD_INPUT, "contact refers to an unknown particle id");
         const bool per = cs->periodic && cs->periodic[r];
-        // P's own entry carries the spring; I's entry carries the same spring for
-        // a direct pair and the reversed one for a periodic pair
-        // (BaseInteraction::copySwitchPointer / reverseHistory).
-        if (!set_entry(sp, si, spr, 1.0) || !set_entry(si, sp, spr, per ? -1.0 : 1.0))
+        // the unit's P is the lower id; the other side of a periodic pair holds
+        // the reversed spring (BaseInteraction::copySwitchPointer / reverseHistory)
+        const bool lower = info[sp].x < info[si].x;
+        if (!set_unit(lower ? sp : si, lower ? si : sp, spr, !lower && per ? -1.0 : 1.0))
             return fail(h, DEM_ERR_BAD_INPUT, "injected contact is not within the neighbour list");
     }
     if (pool.size() / stride > (size_t)d.item_cap)
         return fail(h, DEM_ERR_CAPACITY, "more contact springs than the contact capacity (raise dem_config.max_contacts)");
-    CU(cudaMemcpyAsync(d.act[cur], act.data(), act.size() * sizeof(unsigned), cudaMemcpyHostToDevice, h->stream));
-    CU(cudaMemcpyAsync(d.wact[cur], wact.data(), wact.size() * sizeof(unsigned), cudaMemcpyHostToDevice, h->stream));
-    CU(cudaMemcpyAsync(d.hidx[cur], hidx.data(), hidx.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
+    CU(cudaMemcpyAsync(d.wact[hb], wact.data(), wact.size() * sizeof(unsigned), cudaMemcpyHostToDevice, h->stream));
+    CU(cudaMemcpyAsync(d.uidx[hb], uidx.data(), uidx.size() * sizeof(int), cudaMemcpyHostToDevice, h->stream));
     if (!pool.empty())
         CU(cudaMemcpyAsync(d.pool[c.pcur], pool.data(), pool.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
-    CU(cudaMemcpyAsync(d.whist[cur], whist.data(), whist.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+    CU(cudaMemcpyAsync(d.whist[hb], whist.data(), whist.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
     CU(cudaStreamSynchronize(h->stream));
     return DEM_OK;
 }
@@ -1910,7 +1909,7 @@ int dem_get_counts(dem_handle* hh, int64_t* list_entries, int64_t* contacts, int
     int rc = read_control(h, &c);
     if (rc) return rc;
     std::vector<int> cnt(h->d.n);
-    CU(cudaMemcpyAsync(cnt.data(), h->d.cnt[c.lbuf], cnt.size() * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaMemcpyAsync(cnt.data(), h->d.cnt, cnt.size() * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
     std::vector<ContactRecord> rec(h->records_valid ? h->n_records : 0);
     if (!rec.empty())
         CU(cudaMemcpyAsync(rec.data(), h->d_records, rec.size() * sizeof(ContactRecord), cudaMemcpyDeviceToHost,
@@ -1937,6 +1936,7 @@ int dem_time_force_kernel(dem_handle* hh, int reps, double* ms_per_launch)
     // a mid-batch step: second half-kick, next half-kick and drift, written to
     // the spare buffers; nothing is flipped, so the state stays as it was
     Control probe = saved;
+    probe.spare = 1;
     probe.final_step = 0;
     probe.first_step = 0;
     probe.pending_flip = 0;
@@ -1959,20 +1959,19 @@ int dem_time_force_kernel(dem_handle* hh, int reps, double* ms_per_launch)
 } // extern "C"
 
 namespace {
-// Mean device time of each force kernel (detect, contacts + triangle walls,
-// sum) over `reps` time-step force evaluations on the current state, written
+// Mean device time of each force kernel (units + triangle walls, sum) over `reps` time-step force evaluations on the current state, written
 // to the spare buffers (the probe control of dem_time_force_kernel); the best
 // of three rounds.
-int time_force_parts(Handle* h, int reps, double ms[3])
+int time_force_parts(Handle* h, int reps, double ms[2])
 {
-    std::vector<cudaEvent_t> ev(4 * (size_t)reps);
+    std::vector<cudaEvent_t> ev(3 * (size_t)reps);
     for (auto& e : ev) CU(cudaEventCreate(&e));
-    double best[3] = {1e30, 1e30, 1e30};
+    double best[2] = {1e30, 1e30};
     int rc = DEM_OK;
     launch_force(h, h->stream, 1, false); // warm-up of this shape
     for (int round = 0; round < 3 && rc == DEM_OK; ++round) {
         for (int r = 0; r < reps; ++r) {
-            h->kev = ev.data() + 4 * r;
+            h->kev = ev.data() + 3 * r;
             launch_force(h, h->stream, 1, false);
         }
         h->kev = nullptr;
@@ -1980,18 +1979,18 @@ int time_force_parts(Handle* h, int reps, double ms[3])
             rc = fail(h, DEM_ERR_CUDA, "dem_autotune: a measured launch failed");
             break;
         }
-        double sum[3] = {0, 0, 0};
+        double sum[2] = {0, 0};
         for (int r = 0; r < reps; ++r)
-            for (int k = 0; k < 3; ++k) {
+            for (int k = 0; k < 2; ++k) {
                 float t = 0.f;
-                cudaEventElapsedTime(&t, ev[4 * r + k], ev[4 * r + k + 1]);
+                cudaEventElapsedTime(&t, ev[3 * r + k], ev[3 * r + k + 1]);
                 sum[k] += t;
             }
-        for (int k = 0; k < 3; ++k) best[k] = std::min(best[k], sum[k] / reps);
+        for (int k = 0; k < 2; ++k) best[k] = std::min(best[k], sum[k] / reps);
     }
     h->kev = nullptr;
     for (auto& e : ev) cudaEventDestroy(e);
-    for (int k = 0; k < 3; ++k) ms[k] = best[k];
+    for (int k = 0; k < 2; ++k) ms[k] = best[k];
     return rc;
 }
 
@@ -2016,18 +2015,19 @@ int dem_autotune(dem_handle* hh, int reps, dem_tuning* out)
     int rc = read_control(h, &saved);
     if (rc) return rc;
     Control probe = saved;
+    probe.spare = 1;
     probe.final_step = 0;
     probe.first_step = 0;
     probe.pending_flip = 0;
     probe.record = 0;
     CU(cudaMemcpyAsync(h->d_ctl, &probe, sizeof(Control), cudaMemcpyHostToDevice, h->stream));
     const dem_tuning start = h->tune;
-    double ms[3];
+    double ms[2];
     double before = 0.0;
     if ((rc = time_force_parts(h, reps, ms)) == DEM_OK) {
-        before = ms[0] + ms[1] + ms[2];
-        // one kernel at a time, the others kept: the three kernels share no
-        // launch parameter, and each one's time is measured on its own
+        before = ms[0] + ms[1];
+        // one parameter at a time, the others kept; each kernel's time is
+        // measured on its own
         const int blocks[3] = {64, 128, 256};
         const int per_sm[4] = {3, 4, 5, 6};
         double best = 1e30;
@@ -2044,7 +2044,7 @@ int dem_autotune(dem_handle* hh, int reps, dem_tuning* out)
             if (rc) break;
             h->tune.contacts_blocks_per_sm = b;
             if ((rc = time_force_parts(h, reps, ms))) break;
-            if (ms[1] < best) { best = ms[1]; pick = b; }
+            if (ms[0] < best) { best = ms[0]; pick = b; }
         }
         h->tune.contacts_blocks_per_sm = pick;
         best = 1e30;
@@ -2053,7 +2053,7 @@ int dem_autotune(dem_handle* hh, int reps, dem_tuning* out)
             if (rc) break;
             h->tune.sum_block = b;
             if ((rc = time_force_parts(h, reps, ms))) break;
-            if (ms[2] < best) { best = ms[2]; pick = b; }
+            if (ms[1] < best) { best = ms[1]; pick = b; }
         }
         h->tune.sum_block = pick;
         if (!rc) rc = time_force_parts(h, reps, ms);
@@ -2064,7 +2064,7 @@ int dem_autotune(dem_handle* hh, int reps, dem_tuning* out)
         h->tune = start;
         return rc;
     }
-    const double after = ms[0] + ms[1] + ms[2];
+    const double after = ms[0] + ms[1];
     if (after > before) h->tune = start; // the measurement did not find a faster shape
     h->tune.ms_before = before;
     h->tune.ms_after = std::min(after, before);

@@ -9,21 +9,25 @@
 //   info[b][i] int4    (id, species, instance, flags)
 //   caller[b][i] int   index of the particle in the caller's upload order
 // The 32-byte records let a neighbour's position+radius, velocity+mass and
-// angular velocity+inertia each arrive in one 32-byte sector.
-// Neighbour lists are fixed-capacity rows, one per particle: nbr[l][i*cap + k]
-// (k < count[l][i]); l = Control::lbuf flips at every rebuild. The force
-// kernel walks a warp's entries particle by particle, so a particle's entries
-// are contiguous. Contact history is stored per contact, not per entry: the
-// springs of an evaluation's contacts sit in a pool indexed by the contact's
-// item number in that evaluation, pool[p][j*stride + c] (3 or 9 components
-// per spring, padded), and every list entry keeps the pool index of its
-// contact of the last evaluation, hidx[b][k*ncap + i], valid where its active
-// bit, act[b][w*ncap + i] (bit k%32 of word k/32), is set. hidx and act follow
-// the state buffer b = Control::cur (a rebuild carries them to the new order);
-// the pool flips with every force evaluation (p = Control::pcur: read p,
-// write p^1), and a rebuild leaves it in place. A thread may therefore read its
-// partner's spring of the previous step (needed for periodic pairs) while
-// the partner writes the next one.
+// angular velocity+inertia each arrive in one 32-byte sector. A time step
+// updates the state in place (k_sum touches only its own particle's records);
+// the other buffer takes the permutation of a rebuild.
+//
+// Neighbour lists are fixed-capacity rows, one per particle: rows[i*cap + k]
+// (k < cnt[i]). From them every rebuild makes a flat list of units, the work
+// items of the force evaluation: unit[l][j] = (P, I) is a pair of sorted
+// particle slots with the lower id first, (s, ~w) a particle and a wall w of
+// its instance within reach, (s, UNIT_TRI) a particle near triangle walls. A
+// particle's units are contiguous (from ubase[i]: its pairs in list order,
+// then its walls in wall order), and epair[k*ncap + i] is the unit of its list
+// entry k. Contact history is stored per contact: the springs of an
+// evaluation's contacts sit in a pool indexed by the contact's item number in
+// that evaluation, pool[p][q*stride + c] (3 or 9 components per spring,
+// padded), and every unit keeps the item of its contact of the last
+// evaluation, uidx[h][j] (uidx_kept below). Items also index the force shares
+// that k_units leaves for k_sum. pool and uidx flip with every evaluation
+// (p = Control::pcur, h = Control::hcur: read, write the other); a rebuild
+// carries uidx to the new units (flipping h) and leaves the pool in place.
 #pragma once
 #include <cstdint>
 #include "dem_math.cuh"
@@ -46,6 +50,16 @@ constexpr int FLAG_DORMANT = 4;
 constexpr int FLAG_WRAPPED = 8;
 constexpr double DELETED_COORD = 1e300;
 constexpr int LEVEL_SHIFT = 8;
+
+// I field of a unit for a particle near triangle walls (walls: ~w, w < 32)
+constexpr int UNIT_TRI = INT32_MIN;
+// uidx of a unit: >= 0 the item of its contact; UIDX_NONE no contact and no
+// history; below that a spring kept without a contact (the first time step,
+// k_units), at pool index uidx_kept(v).
+constexpr int UIDX_NONE = -1;
+__host__ __device__ __forceinline__ int uidx_kept(int v) { return -2 - v; }
+// pool index of a unit's spring, -1 if it has none
+__host__ __device__ __forceinline__ int uidx_spring(int v) { return v >= 0 ? v : (v == UIDX_NONE ? -1 : uidx_kept(v)); }
 
 struct InstanceDev {
     double origin[3];
@@ -78,7 +92,7 @@ struct InstanceDev {
     // runs: no translation, and no rotation or one about the wall's own
     // normal / symmetry axis (infinite and axisymmetric walls). The list
     // rebuild records which of them are within reach + skin of a particle
-    // (wcand); k_detect tests the others not at all until the next rebuild
+    // (wcand); the others have no unit until the next rebuild
     uint32_t wall_still_mask;
     // walls (same bits) taken out during the run (WallHandler::removeObject):
     // no contacts with them from the next time step on
@@ -107,18 +121,18 @@ struct ContactRecord {
 
 struct Control {
     int cur;               // state buffer holding the current state
-    int lbuf;              // neighbour-list buffer in use
-    int pending_flip;      // the last force kernel wrote the other state buffer
+    int lbuf;              // unit-list buffer in use
+    int pending_flip;      // the last force evaluation wrote the other spring pool and uidx
     int rebuild;           // this step rebuilds the neighbour list
     int final_step;        // this step is the last of the dem_step call
     int force_rebuild;     // rebuild at the next control point regardless of displacement
     int record;            // record contacts at final/initial evaluations
-    int pad0;
+    int spare;             // 1: k_sum writes the other state buffer (timing launches; the state stays)
     long long steps_left;
     long long n_rebuilds;
     long long steps_done;  // time steps since the upload
     int first_step;        // this step is the first after the initial evaluation
-    int pad1;
+    int hcur;              // uidx (and triangle history) buffer of the last evaluation
     double disp_acc;       // sum of per-step maximum displacements since the last rebuild
     double skin;
     unsigned long long step_disp2_bits; // max |dx|^2 this step (bits of a non-negative double)
@@ -130,6 +144,8 @@ struct Control {
     unsigned int n_tri;    // triangle-wall items of the current evaluation (tri_list)
     int pcur;              // spring pool holding the springs of the last evaluation
     unsigned int n_carry;  // first time step: springs kept without a contact (pool top)
+    int n_units;           // units of the list in use
+    int n_units_next;      // units of the list a rebuild is making
 };
 
 // Entry-major layouts: entry k of every particle is contiguous, so threads
@@ -152,28 +168,29 @@ struct DevPtrs {
     int *caller[2];
     // forces of the last force evaluation (3 per particle, sorted order)
     double *force, *torque;
-    // neighbour lists, two buffers
-    int *nbr[2];
-    int *cnt[2];
-    // ownership bits of list buffer l, laid out like act: bit k%32 of word
-    // own[l][(k/32)*ncap + i] is set when particle i has the lower id of its
-    // entry k's pair (it is P unless the pair meets across a periodic boundary)
-    unsigned int *own[2];
-    // per particle of list buffer l: bit w set when still wall w (above) was
-    // within reach + skin at the rebuild (particles move less than skin / 2
-    // between rebuilds, so the other still walls cannot be touched)
-    unsigned int *wcand[2];
-    double *pool[2];        // springs per contact (item_cap records each)
-    int *hidx[2];           // per entry: pool index of its contact's spring
-    unsigned int *act[2];
-    double *whist[2];
-    unsigned int *wact[2];
+    // neighbour lists of the last rebuild, particle-major
+    int *rows;
+    int *cnt;
+    // ownership bits: bit k%32 of word own[(k/32)*ncap + i] is set when
+    // particle i has the lower id of its entry k's pair
+    unsigned int *own;
+    // walls (bit w = wall_begin + w) particle i has units for: still walls
+    // within reach + skin (particles move less than skin / 2 between
+    // rebuilds, so the others cannot be touched), moving walls, and the
+    // triangle walls its one triangle unit tests
+    unsigned int *wcand;
+    int2 *unit[2];
+    int *uidx[2];
+    int *ubase, *wbase;      // first unit / first wall unit of a particle
+    int *epair;              // per entry: its pair's unit
+    double *pool[2];         // springs per contact (item_cap records each)
+    double *whist[2];        // triangle walls: springs and creation key per (particle, wall)
+    unsigned int *wact[2];   // triangle walls: which of them hold a contact's history
     // broad phase scratch
     int *key, *perm, *newidx, *cell_count, *cell_start, *cell_cursor, *block_sums;
     unsigned long long *rb_barrier; // arrivals at the rebuild's grid barriers (only grows)
     float4 *pf;              // (x, y, z, r) in FP32 of the gathered state: the list build's prefilter
     int *row_slot;           // caller row -> slot of the current order (insertion boundaries only, else null)
-    int *rows;               // neighbour lists particle-major (rows[s * cap + k]), for the reverse index
     // tables
     const InstanceDev *inst;
     const dem_species_pair *species;
@@ -181,19 +198,15 @@ struct DevPtrs {
     const WallGeom *wgeom;   // per wall; faces, edges and corners of intersection walls
     int n_walls;
     int n_instances;
-    // compact contact list of one evaluation (dem_pipeline.cuh)
-    int *rev;                // reverse index of the neighbour lists, n * cap
-    int *slot;               // per entry: item index, or SLOT_NONE / SLOT_IS_I
-    int *slotw;              // per (particle, wall): item index or SLOT_NONE
-    int4 *items;             // (particle, entry or ITEM_WALL + wall, partner slot, 0);
-                             // (particle, ITEM_TRI, triangle-wall hit bits, 0)
-    int *tri_list;           // item index of each triangle-wall item (n_tri of them)
-    int *slott;              // per particle: its triangle-wall item or SLOT_NONE
+    // triangle-wall items of one evaluation: (particle, item, wall bits, 0)
+    int4 *tri_list;
+    int *slott;              // per particle: its triangle-wall item or -1
     double *tri_first;       // triangle contacts of the initial evaluation, TRI_REC doubles each,
                              // DEM_MAX_TRIANGLE_CONTACTS per particle in caller order (k_tri)
     int *tri_first_n;        // their number per particle (caller order)
-    double *shares;          // 12 doubles per item
+    double *shares;          // 12 doubles per item: P force, P torque, I force, I torque
     int item_cap;
+    int unit_cap;
     Control *ctl;
     ContactRecord *records;
     // sizes
@@ -201,11 +214,12 @@ struct DevPtrs {
     int ncap;         // allocated particle slots (ELL stride)
     int cap;          // neighbour capacity per particle (multiple of 32)
     int nwords;       // cap / 32
+    int any_periodic; // some instance has a periodic direction
     int ncomp;        // history components per contact (3 or 9)
     int wmax;         // max walls per instance
     int ncells;
     int rotation;
-    int single_instance;   // one instance: k_contacts stages its record in shared memory
+    int single_instance;   // one instance: k_units stages its record in shared memory
     int n_species_table;   // entries of the species table
     int zero_idist;        // every species pair has interaction distance 0
     int has_tri;           // some wall is a triangle wall (k_tri runs)

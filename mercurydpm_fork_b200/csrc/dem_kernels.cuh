@@ -13,14 +13,13 @@
 //               contact-history carry-over, their reverse index (replaces
 //               HGrid buckets + InteractionHandler lookup, Mercury3D.cc:224-416,
 //               InteractionHandler.cc:103-174). The per-item steps are below.
-//   force       k_detect -> k_contacts -> k_sum (dem_pipeline.cuh): the exact
-//               FP64 contact predicate (BaseParticle::getInteractionWith,
-//               BaseParticle.cc:688-710) on the entries each particle owns,
-//               the contact law once per contact with its spring history,
-//               the ordered sums with body force and walls, and the
-//               integration (second half-kick of this step, then first
-//               half-kick and drift of the next one: BaseParticle.cc:718-776)
-//               into the other state buffer.
+//   force       k_units -> k_sum (dem_pipeline.cuh): the exact FP64 contact
+//               predicate (BaseParticle::getInteractionWith,
+//               BaseParticle.cc:688-710) and the contact law once per contact
+//               with its spring history, then the ordered sums with body
+//               force and walls, and the integration (second half-kick of
+//               this step, then first half-kick and drift of the next one:
+//               BaseParticle.cc:718-776), in place.
 #pragma once
 #include "dem_engine.cuh"
 #include "dem_laws.cuh"
@@ -52,8 +51,8 @@ __global__ void k_control(Control* ctl, dem_wall* walls, WallGeom* wgeom, int n_
         if (w.type == DEM_WALL_TRIANGLE && !still) triangle_geometry(w, wgeom[k]);
     }
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (ctl->pending_flip) { // a force evaluation wrote the other state buffer and spring pool
-        ctl->cur ^= 1;
+    if (ctl->pending_flip) { // a force evaluation wrote the other spring pool and uidx
+        ctl->hcur ^= 1;
         ctl->pcur ^= 1;
         ctl->pending_flip = 0;
     }
@@ -68,14 +67,14 @@ __global__ void k_control(Control* ctl, dem_wall* walls, WallGeom* wgeom, int n_
     if (ctl->final_step) ctl->n_records = 0; // records describe the last evaluation only
     ctl->first_step = (ctl->steps_done == 0);
     ctl->steps_done += 1;
-    ctl->pending_flip = 1; // the force kernel of this step writes the other buffer
+    ctl->pending_flip = 1; // the force evaluation of this step writes the other pool
 }
 
 __global__ void k_flip(Control* ctl)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (ctl->pending_flip) { // a force evaluation wrote the other state buffer and spring pool
-        ctl->cur ^= 1;
+    if (ctl->pending_flip) { // a force evaluation wrote the other spring pool and uidx
+        ctl->hcur ^= 1;
         ctl->pcur ^= 1;
         ctl->pending_flip = 0;
     }
@@ -236,17 +235,6 @@ __device__ __forceinline__ int wrap_cell(int c, int dim)
     return c < 0 ? c + dim : c;
 }
 
-// Sets bit m of a 4-word mask held in registers.
-__device__ __forceinline__ void set_bit4(unsigned int& w0, unsigned int& w1, unsigned int& w2, unsigned int& w3, int m)
-{
-    const unsigned int bit = 1u << (m & 31);
-    const int w = m >> 5;
-    if (w == 0) w0 |= bit;
-    else if (w == 1) w1 |= bit;
-    else if (w == 2) w2 |= bit;
-    else w3 |= bit;
-}
-
 // Slot ranges of one (z, y) row of cells between x cells lo..hi: one range,
 // or two when a periodic row wraps (the second empty otherwise).
 __device__ __forceinline__ void row_ranges(const DevPtrs& d, const InstanceDev& I, int lvl, int row, int lo, int hi,
@@ -273,6 +261,20 @@ __device__ __forceinline__ void row_ranges(const DevPtrs& d, const InstanceDev& 
     }
 }
 
+// The tests that open TriangleWall::getDistanceAndNormal, with reach R: inside
+// the vertices' bounding box widened by R (the region the reference searches,
+// Mercury3D::computeWallForces with TriangleWall::isLocal), and near the face
+// plane.
+__device__ __forceinline__ bool triangle_near(const WallGeom& tg, V3 x, double R)
+{
+    return x.x > tg.tlo[0] - R && x.x < tg.thi[0] + R && x.y > tg.tlo[1] - R && x.y < tg.thi[1] + R &&
+           x.z > tg.tlo[2] - R && x.z < tg.thi[2] + R;
+}
+__device__ __forceinline__ bool triangle_plane_near(const WallGeom& tg, V3 x, double R)
+{
+    return fabs(dot(x - row3(tg.tv[0]), row3(tg.tfn))) < R;
+}
+
 // Neighbour list of one particle: every particle of the cells within reach
 // whose distance is below r_s + r_t + interaction distance + skin, in
 // cell-row order. The distance test runs in FP32 on the `pf` copy
@@ -284,22 +286,20 @@ __device__ __forceinline__ void row_ranges(const DevPtrs& d, const InstanceDev& 
 // take the FP64 test. Contacts themselves are always decided in FP64
 // by the force evaluation, so the superset changes no result. The next row's
 // slot ranges are read ahead and candidates are read BUILD_BATCH at a time.
+// Also the walls of the particle's units (wcand). `pairs` gets the entries the
+// particle owns (one unit each), `walls` its wall units.
 constexpr int BUILD_BATCH = 2;
-__device__ __forceinline__ void build_one(const DevPtrs& d, int s, int hc, int lo_)
+__device__ __forceinline__ void build_one(const DevPtrs& d, int s, int nb, int& pairs, int& walls)
 {
-    // hc: old state order and its history; lo_: old lists
-    const int nb = hc ^ 1;             // gathered (new) state; new history
-    const int ln = lo_ ^ 1;            // new lists
-    const double4 ps = d.pr[nb][s];
+    const double4 ps = d.pr[nb][s]; // the gathered state
     const int4 is = d.info[nb][s];
     const InstanceDev& I = d.inst[is.z];
     const V3 xs = xyz(ps);
     const bool fixed_s = (is.w & FLAG_FIXED) != 0;
+    pairs = walls = 0;
     if (is.w & FLAG_DELETED) {
-        d.cnt[ln][s] = 0;
-        d.wcand[ln][s] = 0u;
-        for (int w = 0; w < d.nwords; ++w) d.act[nb][(size_t)w * d.ncap + s] = 0u;
-        d.wact[nb][s] = 0u;
+        d.cnt[s] = 0;
+        d.wcand[s] = 0u;
         return;
     }
     const double extra = I.max_interaction_distance + d.ctl->skin;
@@ -386,11 +386,14 @@ __device__ __forceinline__ void build_one(const DevPtrs& d, int s, int hc, int l
                         }
                         if (near) {
                             if (count < d.cap) {
-                                d.nbr[ln][nbr_at(d.ncap, s, count)] = t;
                                 d.rows[(size_t)s * d.cap + count] = t;
-                                if (is.x < d.info[nb][t].x) ownw |= 1u << (count & 31);
+                                d.epair[nbr_at(d.ncap, s, count)] = -1; // its unit, once made (units_one)
+                                if (is.x < d.info[nb][t].x) {
+                                    ownw |= 1u << (count & 31);
+                                    ++pairs;
+                                }
                                 if ((count & 31) == 31) {
-                                    d.own[ln][(size_t)(count >> 5) * d.ncap + s] = ownw;
+                                    d.own[(size_t)(count >> 5) * d.ncap + s] = ownw;
                                     ownw = 0u;
                                 }
                             } else {
@@ -407,93 +410,58 @@ __device__ __forceinline__ void build_one(const DevPtrs& d, int s, int hc, int l
         atomicOr(&d.ctl->status, 1u << DEM_ERR_CAPACITY);
         count = d.cap;
     }
-    if (count & 31) d.own[ln][(size_t)(count >> 5) * d.ncap + s] = ownw; // the last, partial word
-    d.cnt[ln][s] = count;
+    if (count & 31) d.own[(size_t)(count >> 5) * d.ncap + s] = ownw; // the last, partial word
+    d.cnt[s] = count;
 
-    // still walls within reach + skin (k_detect tests only these until the next rebuild)
-    unsigned int wc = 0u;
+    // the walls to test until the next rebuild: still walls within reach +
+    // skin, the other ones always. Triangle walls that stand still: the test
+    // of k_units (bounding box, face plane) with the reach widened by the skin,
+    // which leaves more than the skin / 2 a particle moves between rebuilds.
+    unsigned int wc = 0u, tris = 0u;
     if (!fixed_s) {
         const int nwl = I.wall_end - I.wall_begin;
+        const double skin = d.ctl->skin;
         for (int w = 0; w < nwl; ++w) {
-            if (!((I.wall_still_mask >> w) & 1u)) continue;
+            const unsigned int bit = 1u << w;
+            if (I.wall_off_mask & bit) continue;
             const int wg = I.wall_begin + w;
-            const dem_wall& wall = d.walls[wg];
-            const double R = ps.w + d.species[I.species_offset + is.y * I.n_species + wall.species].interaction_distance +
-                             d.ctl->skin;
-            double dist;
-            V3 nrm;
-            if (wall_distance(wall, d.wgeom + wg, xs, R, dist, nrm)) wc |= 1u << w;
+            if (I.tri_mask & bit) {
+                const WallGeom& tg = d.wgeom[wg];
+                const double R = (ps.w + I.max_interaction_distance + skin) * (1.0 + 1e-12);
+                if (!I.tri_static || (triangle_near(tg, xs, R) && triangle_plane_near(tg, xs, R))) tris |= bit;
+                continue;
+            }
+            if ((I.wall_still_mask >> w) & 1u) {
+                const dem_wall& wall = d.walls[wg];
+                const double R = ps.w + d.species[I.species_offset + is.y * I.n_species + wall.species].interaction_distance +
+                                 skin;
+                double dist;
+                V3 nrm;
+                if (!wall_distance(wall, d.wgeom + wg, xs, R, dist, nrm)) continue;
+            }
+            wc |= bit;
+            ++walls;
         }
     }
-    d.wcand[ln][s] = wc;
+    if (tris) ++walls;
+    d.wcand[s] = wc | tris;
+}
 
-    // carry contact history from the old list (old order) to the new one, up
-    // to 4 contacts per pass over the new list
+// Triangle-wall history of slot s moves with its particle (h: the buffer
+// read, the other one written; c: the state buffer of the old order): springs
+// and, in the pad word, the creation key (k_tri).
+__device__ __forceinline__ void carry_triangles(const DevPtrs& d, int s, int h, int c)
+{
     const int o = d.perm[s];
-    const int ocnt = d.cnt[lo_][o];
-    unsigned int n0 = 0u, n1 = 0u, n2 = 0u, n3 = 0u;
-    for (int w = 0; w < d.nwords; ++w) {
-        unsigned int bits = d.act[hc][(size_t)w * d.ncap + o];
-        while (bits) {
-            int kk[4], tn[4], m[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                kk[j] = -1;
-                if (bits) {
-                    const int k = w * 32 + __ffs(bits) - 1;
-                    bits &= bits - 1;
-                    if (k < ocnt) kk[j] = k; // bits past the old count are stale
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) tn[j] = kk[j] >= 0 ? d.nbr[lo_][nbr_at(d.ncap, o, kk[j])] : -1;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                tn[j] = tn[j] >= 0 ? d.newidx[tn[j]] : -1;
-                m[j] = -1;
-            }
-            for (int q0 = 0; q0 < count; q0 += 4) {
-                int v[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) v[i] = (q0 + i < count) ? d.nbr[ln][nbr_at(d.ncap, s, q0 + i)] : -2;
-#pragma unroll
-                for (int j = 0; j < 4; ++j)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        if (m[j] < 0 && tn[j] >= 0 && v[i] == tn[j]) m[j] = q0 + i;
-                bool done = true;
-#pragma unroll
-                for (int j = 0; j < 4; ++j) done = done && (tn[j] < 0 || m[j] >= 0);
-                if (done) break;
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                if (kk[j] < 0) continue;
-                if (m[j] < 0) {
-                    atomicAdd(&d.ctl->lost_history, 1u);
-                    continue;
-                }
-                // the spring stays where it is in the pool; the new entry points at it
-                d.hidx[nb][nbr_at(d.ncap, s, m[j])] = d.hidx[hc][nbr_at(d.ncap, o, kk[j])];
-                set_bit4(n0, n1, n2, n3, m[j]);
-            }
-        }
-    }
-    const unsigned int nw[4] = {n0, n1, n2, n3};
-#pragma unroll
-    for (int w = 0; w < 4; ++w)
-        if (w < d.nwords) d.act[nb][(size_t)w * d.ncap + s] = nw[w];
-    // wall history moves with the particle (with the pad word: a triangle
-    // contact's creation key, k_tri)
-    const unsigned int wbits = d.wact[hc][o];
-    d.wact[nb][s] = wbits;
-    unsigned int bits = wbits;
-    while (bits) {
+    const int4 is = d.info[c][o];
+    const unsigned int tri = (is.w & FLAG_DELETED) ? 0u : d.inst[is.z].tri_mask & d.wcand[s];
+    const unsigned int keep = d.wact[h][o] & tri;
+    d.wact[h ^ 1][s] = keep;
+    d.slott[s] = -1;
+    for (unsigned int bits = keep; bits; bits &= bits - 1) {
         const int w = __ffs(bits) - 1;
-        bits &= bits - 1;
-        for (int comp = 0; comp < d.ncomp; ++comp)
-            d.whist[nb][whist_at(d.ncap, d.ncomp, s, w) + comp] = d.whist[hc][whist_at(d.ncap, d.ncomp, o, w) + comp];
-        if (d.has_tri) d.whist[nb][whist_at(d.ncap, d.ncomp, s, w) + d.ncomp] = d.whist[hc][whist_at(d.ncap, d.ncomp, o, w) + d.ncomp];
+        for (int q = 0; q < hist_stride(d.ncomp); ++q)
+            d.whist[h ^ 1][whist_at(d.ncap, d.ncomp, s, w) + q] = d.whist[h][whist_at(d.ncap, d.ncomp, o, w) + q];
     }
 }
 

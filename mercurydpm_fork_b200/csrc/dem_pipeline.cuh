@@ -1,57 +1,53 @@
-// dem_pipeline.cuh -- one force evaluation as three kernels over a compact
-// contact list, each contact's law evaluated once:
+// dem_pipeline.cuh -- one force evaluation as two kernels over the flat unit
+// list of the last rebuild (pairs with the lower id first, particle-wall
+// candidates), each contact's law evaluated once:
 //
-//   k_detect   one thread per particle: the exact contact predicate
-//              (BaseParticle::getInteractionWith, BaseParticle.cc:688-710) on
-//              the neighbour entries the particle owns as P -- the lower id,
-//              or its own view of a periodic pair (DPMBase.cc:3124-3139) --
-//              and on its walls; contacts are appended to a compact item list
-//              (one atomic per block) and every entry gets its item index or a
-//              role mark; history bits of the next buffer are written here.
-//   k_contacts one thread per contact item: the contact law with the spring
-//              history (DPMBase::computeInternalForce, DPMBase.cc:3113-3162;
-//              walls: DPMBase.cc:3188-3215), the force/torque share of P and,
-//              for an ordinary pair, of I, into the item's 12 doubles.
+//   k_units    persistent blocks, a chunk of units at a time: the exact contact
+//              predicate (BaseParticle::getInteractionWith,
+//              BaseParticle.cc:688-710), one unit per thread with several in
+//              flight; the block's contacts, compacted in shared memory, then
+//              take the contact law with full warps (DPMBase::
+//              computeInternalForce, DPMBase.cc:3113-3162; walls:
+//              DPMBase.cc:3188-3215) with the spring of the unit's last
+//              contact, and leave the force/torque shares of P and I at their
+//              item. A pair that meets across a periodic boundary is two views,
+//              each real particle against the other's ghost
+//              (DPMBase.cc:3124-3139), evaluated by the same thread.
 //   k_tri      (only with triangle walls) one thread per particle with
-//              triangle-wall candidates: the reference's wall loop for them
-//              with group merging and overlap weighting, into one item.
-//   k_sum      one thread per particle: the shares in neighbour-list order
-//              (P entries from its own items, I entries from the partner's
-//              item, which k_contacts announces in I's entry through the
-//              reverse index), the body force
-//              (DPMBase.cc:3168-3179), then the wall shares -- the order the
-//              sequential code adds them -- then the integration tail.
+//              triangle-wall contacts in reach: the reference's wall loop for
+//              them with group merging and overlap weighting, into one item.
+//   k_sum      one thread per particle: the shares in neighbour-list order,
+//              the body force (DPMBase.cc:3168-3179), then the wall shares --
+//              the order the sequential code adds them -- then the
+//              integration.
 //
-// The entry and item orders do not change any sum: each particle adds its
-// shares in its own list order, so results are independent of the atomics.
+// Items are numbered by atomics; each particle adds its shares in its own
+// list order, so results do not depend on them.
+//
 #pragma once
 #include "dem_kernels.cuh"
 
 namespace dem {
 
-constexpr int ITEM_WALL = 1 << 20;   // item entry field >= this: wall contact (ITEM_WALL + wall)
-constexpr int ITEM_TRI = ITEM_WALL + (1 << 10); // all triangle-wall contacts of a particle (k_tri)
 // One triangle contact of the initial evaluation (k_tri): wall, creation key,
 // overlap, normal, force, torque, contact point, species, normal elastic
 // energy, springs.
 constexpr int TRI_REC = 26;
-constexpr int SLOT_NONE = -1;        // P entry without a contact this evaluation
-constexpr int SLOT_IS_I = -2;        // entry whose partner owns the pair, no contact this evaluation
-constexpr int SLOT_I_BASE = -3;      // SLOT_I_BASE - q: I's share of the partner's item q
 constexpr int SHARE = 12;            // doubles per item: P force, P torque, I force, I torque
-// Launch shapes. k_detect and k_sum are compiled for blocks of 64, 128 and
-// 256 threads and k_contacts' grid size is a run-time value; the handle keeps
-// the choice (dem_autotune measures the variants on the live state).
-constexpr int DETECT_BLOCK = 128;        // the default k_detect block
-constexpr int CONTACT_BLOCK = 128;
+// Launch shapes. k_units is compiled for 3 to 6 resident blocks per SM and
+// k_sum for blocks of 64, 128 and 256 threads; the handle keeps the choice
+// (dem_autotune measures the variants on the live state).
+constexpr int UNIT_BLOCK = 128;
+constexpr int UNIT_CHUNK_PER_TUNE = 4;   // units a block takes at a time: at most 4 x dem_tuning.detect_block
+constexpr int UNIT_CHUNK_MAX = 256 * UNIT_CHUNK_PER_TUNE;
+constexpr int DETECT_TUNE = 128;         // the default dem_tuning.detect_block
 constexpr int SUM_BLOCK = 128;           // the default k_sum block
 constexpr int SUM_THREADS_PER_SM = 640;  // k_sum's launch bounds: 640 / block resident blocks per SM
 
 // Shared-memory copies of the instance record (when there is one instance)
 // and of the species-pair table (when it has at most SP_STAGE_MAX entries),
-// staged by k_contacts' blocks before their first item: the contact law's
-// parameters are then no dependent global loads (measured: 51.6 -> 49.1 us per
-// evaluation on the 200k chute; k_detect and k_sum gained nothing from it).
+// staged by k_units' blocks before their first contact: the contact law's
+// parameters are then no dependent global loads.
 constexpr int SP_STAGE_MAX = 16;
 struct TableStage {
     __align__(16) unsigned char inst[sizeof(InstanceDev)];
@@ -59,7 +55,8 @@ struct TableStage {
 };
 static_assert(sizeof(InstanceDev) % 4 == 0 && sizeof(dem_species_pair) % 4 == 0, "staged as 32-bit words");
 
-// Called by every thread of the block (it synchronises the block).
+// Called by every thread of the block; the copies are there after the block's
+// next barrier.
 __device__ __forceinline__ void stage_tables(const DevPtrs& d, TableStage& st)
 {
     if (d.single_instance) {
@@ -73,7 +70,6 @@ __device__ __forceinline__ void stage_tables(const DevPtrs& d, TableStage& st)
         const int words = d.n_species_table * (int)(sizeof(dem_species_pair) / 4);
         for (int k = threadIdx.x; k < words; k += blockDim.x) dst[k] = src[k];
     }
-    __syncthreads();
 }
 
 __device__ __forceinline__ const InstanceDev& staged_inst(const DevPtrs& d, const TableStage& st, int z)
@@ -107,38 +103,118 @@ __device__ __forceinline__ int find_in_row(const DevPtrs& d, int s, int t, int c
     return -1;
 }
 
-// Reverse index of one particle's list (after a rebuild, lists buffer l):
-// rev[s][k] = m with nbr[t][m] == s for t = nbr[s][k] (the lists are
-// symmetric). Two entries at a time; the partners' rows are read from the
-// particle-major copy that build_one writes (the first 16 entries of both
-// rows in flight together). Run by k_rebuild.
-__device__ __forceinline__ void rev_one(const DevPtrs& d, int s, int l)
+// Number of entries before k that particle s owns (the rank of entry k's pair
+// among its units).
+__device__ __forceinline__ int own_rank(const DevPtrs& d, int s, int k)
 {
-    const int cnt = min(d.cnt[l][s], d.cap);
-    for (int k0 = 0; k0 < cnt; k0 += 2) {
-        int t[2], ct[2];
-        int4 head[2][4];
+    int r = 0;
+    for (int w = 0; w < (k >> 5); ++w) r += __popc(d.own[(size_t)w * d.ncap + s]);
+    return r + __popc(d.own[(size_t)(k >> 5) * d.ncap + s] & ((1u << (k & 31)) - 1u));
+}
+
+// The units of particle s after a rebuild (list buffer l, uidx buffer h, state
+// buffer nb): its own pairs, each filed in both particles' entries (the partner's row is
+// searched for s; the lists are symmetric), two at a time with the first 16
+// entries of both rows in flight together, then its walls. None has a
+// history yet.
+__device__ __forceinline__ void units_one(const DevPtrs& d, int s, int l, int h, int nb)
+{
+    const int cnt = min(d.cnt[s], d.cap);
+    const int base = d.ubase[s];
+    int u = base, pairs = 0;
+    for (int w = 0; 32 * w < cnt; ++w) {
+        const int left = cnt - 32 * w;
+        unsigned int todo = d.own[(size_t)w * d.ncap + s] & (left >= 32 ? 0xffffffffu : (1u << left) - 1u);
+        pairs += __popc(todo);
+        while (todo) {
+            int t[2], ct[2], k[2];
+            int4 head[2][4];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) t[j] = (k0 + j < cnt) ? d.nbr[l][nbr_at(d.ncap, s, k0 + j)] : -1;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-            if (t[j] >= 0) {
-                ct[j] = d.cnt[l][t[j]];
-                const int4* row = reinterpret_cast<const int4*>(d.rows + (size_t)t[j] * d.cap);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) head[j][q] = row[q]; // 16 <= cap entries: inside the row
+            for (int j = 0; j < 2; ++j) {
+                t[j] = -1;
+                if (todo) {
+                    k[j] = 32 * w + __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    t[j] = d.rows[(size_t)s * d.cap + k[j]];
+                }
             }
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            if (t[j] < 0) continue;
-            int m = find_in_row(d, s, t[j], min(ct[j], d.cap), head[j]);
-            if (m < 0) {
-                atomicOr(&d.ctl->status, 1u << DEM_ERR_CAPACITY); // an asymmetric pair: the partner's row overflowed
-                m = 0;
+            for (int j = 0; j < 2; ++j)
+                if (t[j] >= 0) {
+                    ct[j] = d.cnt[t[j]];
+                    const int4* row = reinterpret_cast<const int4*>(d.rows + (size_t)t[j] * d.cap);
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) head[j][q] = row[q]; // 16 <= cap entries: inside the row
+                }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if (t[j] < 0) continue;
+                const int m = find_in_row(d, s, t[j], min(ct[j], d.cap), head[j]);
+                // an asymmetric pair (the partner's row overflowed) or too many of them: no unit
+                if (m < 0 || (unsigned)u >= (unsigned)d.unit_cap) {
+                    atomicOr(&d.ctl->status, 1u << DEM_ERR_CAPACITY);
+                    continue;
+                }
+                d.epair[nbr_at(d.ncap, t[j], m)] = u;
+                d.epair[nbr_at(d.ncap, s, k[j])] = u;
+                d.unit[l][u] = make_int2(s, t[j]);
+                d.uidx[h][u] = UIDX_NONE;
+                ++u;
             }
-            d.rev[nbr_at(d.ncap, s, k0 + j)] = m;
         }
     }
+    for (; u < base + pairs; ++u) // units of pairs left out above
+        if ((unsigned)u < (unsigned)d.unit_cap) {
+            d.unit[l][u] = make_int2(-1, -1);
+            d.uidx[h][u] = UIDX_NONE;
+        }
+    const unsigned int mask = d.wcand[s];
+    d.wbase[s] = u;
+    if (!mask) return;
+    const unsigned int tri = d.has_tri ? d.inst[d.info[nb][s].z].tri_mask : 0u;
+    const int n_walls = __popc(mask & ~tri) + ((mask & tri) ? 1 : 0);
+    if ((unsigned)u + n_walls > (unsigned)d.unit_cap) {
+        atomicOr(&d.ctl->status, 1u << DEM_ERR_CAPACITY);
+        d.wcand[s] = 0u;
+        return;
+    }
+    for (unsigned int b = mask & ~tri; b; b &= b - 1, ++u) {
+        d.unit[l][u] = make_int2(s, ~(__ffs(b) - 1));
+        d.uidx[h][u] = UIDX_NONE;
+    }
+    if (mask & tri) {
+        d.unit[l][u] = make_int2(s, UNIT_TRI);
+        d.uidx[h][u] = UIDX_NONE;
+    }
+}
+
+// The history of old unit j (list buffer l, uidx buffer h, state buffer c)
+// moves to the same pair or wall of the new list.
+__device__ __forceinline__ void carry_one(const DevPtrs& d, int j, int l, int h, int c)
+{
+    const int v = d.uidx[h][j];
+    if (v == UIDX_NONE) return;
+    const int2 old = d.unit[l][j];
+    if (old.x < 0 || old.y == UNIT_TRI) return; // a triangle history moves with the particle (carry_triangles)
+    const int s = d.newidx[old.x];
+    int u = -1;
+    if (old.y >= 0) {
+        const int t = d.newidx[old.y];
+        const int ct = min(d.cnt[s], d.cap);
+        const int4* row = reinterpret_cast<const int4*>(d.rows + (size_t)s * d.cap);
+        int4 head[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) head[q] = row[q];
+        const int m = find_in_row(d, t, s, ct, head);
+        if (m >= 0) u = d.ubase[s] + own_rank(d, s, m);
+        else atomicAdd(&d.ctl->lost_history, 1u); // out of reach, or deleted
+    } else {
+        const unsigned int bit = 1u << ~old.y, mask = d.wcand[s];
+        const unsigned int tri = d.has_tri ? d.inst[d.info[c][old.x].z].tri_mask : 0u;
+        if (mask & bit) u = d.wbase[s] + __popc(mask & ~tri & (bit - 1u));
+    }
+    // the spring stays where it is in the pool; the new unit points at it
+    if (u >= 0 && (unsigned)u < (unsigned)d.unit_cap) d.uidx[h ^ 1][u] = v;
 }
 
 // Exclusive block scan of one int per thread (any block of whole warps); returns
@@ -163,231 +239,85 @@ __device__ __forceinline__ int block_exclusive_scan(int v, int* warp_sums, int& 
     return before + x - v;
 }
 
-template <int MODE, int NCOMP, int BLOCK>
-__global__ void __launch_bounds__(BLOCK) k_detect(DevPtrs d)
+// What the first time step does with a unit that had a contact in the initial
+// evaluation and has none now: the interaction outlives the step
+// (InteractionHandler::eraseOldInteractions erases stamps <= 0 only), so its
+// spring moves to the top of the next pool, below which the items of this
+// evaluation stay (k_sum checks that they met no carry).
+template <int NCOMP>
+__device__ __forceinline__ int keep_spring(const DevPtrs& d, int pc, int from_idx)
 {
-    constexpr int HIT_KEEP = 16; // partner slots of the first hits, kept for the item pass
-    __shared__ int warp_sums[BLOCK / 32];
-    __shared__ int block_base;
-    __shared__ int kept_t[HIT_KEEP][BLOCK];
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    Control* ctl = d.ctl;
-    const int c = ctl->cur, l = ctl->lbuf, nb = c ^ 1, pc = ctl->pcur;
-    const bool first = (MODE == 1) && ctl->first_step;
-    const bool active = s < d.n;
-    // hit bits of the (at most 4) list words, in registers: each word is
-    // finished before the next starts, so no dynamically indexed array
-    unsigned int hit0 = 0u, hit1 = 0u, hit2 = 0u, hit3 = 0u;
-    int nkept = 0;
-    unsigned int whit = 0u, wnew = 0u, thit = 0u;
-    int count = 0, nwalls = 0;
-    if (active) {
-        const double4 ps = d.pr[c][s];
-        const int4 is = d.info[c][s];
-        const InstanceDev& I = d.inst[is.z];
-        const V3 xs = xyz(ps);
-        count = min(d.cnt[l][s], d.cap);
-        const int ns = I.n_species;
-        constexpr int B = 2; // entries whose gathers are in flight together (2 keeps 80 registers)
-        const int2* info2 = reinterpret_cast<const int2*>(d.info[c]); // (id, species) of each info record
-        // Without periodic boundaries a pair's owner (the lower id) is fixed
-        // for the life of a list, and the rebuild stored it (own bits): the
-        // partner-owned entries are marked without gathering the partner, and
-        // the owned ones are visited in list order, B at a time. With periodic
-        // boundaries every entry is visited (its image decides the owner).
-        const bool owner_known = I.per_mask == 0u;
-        for (int w = 0; w < d.nwords; ++w) {
-            unsigned int hitw = 0u, neww = 0u;
-            const int kbeg = 32 * w, kend = min(count, kbeg + 32);
-            const unsigned int valid = kend <= kbeg ? 0u : (kend - kbeg == 32 ? 0xffffffffu : (1u << (kend - kbeg)) - 1u);
-            unsigned int todo = valid;
-            if (owner_known && valid) {
-                const unsigned int ow = d.own[l][(size_t)w * d.ncap + s];
-                unsigned int other = valid & ~ow;
-                while (other) {
-                    const int k = kbeg + __ffs(other) - 1;
-                    other &= other - 1;
-                    d.slot[nbr_at(d.ncap, s, k)] = SLOT_IS_I;
-                }
-                todo = valid & ow;
-            }
-            const unsigned int aw = (first && valid) ? d.act[c][(size_t)w * d.ncap + s] : 0u;
-            while (todo) {
-                int kb[B], tb[B];
-                double4 ptb[B];
-                int2 itb[B];
-#pragma unroll
-                for (int j = 0; j < B; ++j) {
-                    kb[j] = -1;
-                    if (todo) {
-                        kb[j] = kbeg + __ffs(todo) - 1;
-                        todo &= todo - 1;
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < B; ++j) tb[j] = kb[j] >= 0 ? d.nbr[l][nbr_at(d.ncap, s, kb[j])] : -1;
-#pragma unroll
-                for (int j = 0; j < B; ++j)
-                    if (tb[j] >= 0) {
-                        ptb[j] = d.pr[c][tb[j]];
-                        itb[j] = info2[2 * (size_t)tb[j]];
-                    }
-#pragma unroll
-                for (int j = 0; j < B; ++j) {
-                    const int k = kb[j];
-                    if (k < 0) break;
-                    const size_t e = nbr_at(d.ncap, s, k);
-                    const double4 pt = ptb[j];
-                    const int2 it = itb[j];
-                    bool periodic;
-                    const V3 xt = image_of(I, xs, xyz(pt), periodic);
-                    if (!periodic && !(is.x < it.x)) { // the partner (lower id) owns this pair
-                        d.slot[e] = SLOT_IS_I;
-                        continue;
-                    }
-                    d.slot[e] = SLOT_NONE;
-                    const V3 branch = xs - xt;
-                    const double d2 = len2(branch);
-                    double idist = 0.0; // x + 0.0 == x: skipping the lookup keeps the predicate exact
-                    if (!d.zero_idist) idist = d.species[I.species_offset + is.y * ns + it.y].interaction_distance;
-                    const double sum = pt.w + ps.w + idist; // rI + rP + distance (BaseParticle.cc:695-697)
-                    const unsigned int bit = 1u << (k & 31);
-                    if (!(d2 >= sum * sum)) {
-                        hitw |= bit;
-                        if (nkept < HIT_KEEP) kept_t[nkept++][threadIdx.x] = tb[j];
-                        neww |= bit;
-                    } else if (first && (aw & bit) && !(periodic && is.x > it.x)) {
-                        // an interaction of the initial evaluation outlives step 0
-                        // (InteractionHandler::eraseOldInteractions erases stamps <= 0 only):
-                        // its spring moves to the top of the next pool, below which the
-                        // items of this evaluation stay (k_sum checks that they met no carry)
-                        const int top = d.item_cap - 1 - (int)atomicAdd(&ctl->n_carry, 1u);
-                        if (top >= 0) {
-                            const double2* from = reinterpret_cast<const double2*>(d.pool[pc] + pool_at(NCOMP, d.hidx[c][e]));
-                            double2* to = reinterpret_cast<double2*>(d.pool[pc ^ 1] + pool_at(NCOMP, top));
-#pragma unroll
-                            for (int q = 0; q < hist_stride(NCOMP) / 2; ++q) to[q] = from[q];
-                            d.hidx[nb][e] = top;
-                            neww |= bit;
-                        } else {
-                            atomicOr(&ctl->status, 1u << DEM_ERR_CAPACITY);
-                        }
-                    }
-                }
-            }
-            d.act[nb][(size_t)w * d.ncap + s] = neww;
-            if (w == 0) hit0 = hitw;
-            else if (w == 1) hit1 = hitw;
-            else if (w == 2) hit2 = hitw;
-            else hit3 = hitw;
-        }
-        if (!(is.w & FLAG_FIXED)) {
-            const unsigned int wa = d.wact[c][s];
-            nwalls = I.wall_end - I.wall_begin;
-            bool near_tri = false; // within reach of the instance's triangles (all of them, if they move)
-            if (d.has_tri && I.tri_mask) {
-                d.slott[s] = SLOT_NONE;
-                // widened by a relative 1e-12 so that rounding of tri_lo - R cannot
-                // skip a particle at exactly the reach
-                const double R = (ps.w + I.max_interaction_distance) * (1.0 + 1e-12);
-                near_tri = !I.tri_static ||
-                           (xs.x > I.tri_lo[0] - R && xs.x < I.tri_hi[0] + R && xs.y > I.tri_lo[1] - R &&
-                            xs.y < I.tri_hi[1] + R && xs.z > I.tri_lo[2] - R && xs.z < I.tri_hi[2] + R);
-            }
-            // farther than reach + skin at the last rebuild, or taken out
-            const unsigned int far_still = (I.wall_still_mask & ~d.wcand[l][s]) | I.wall_off_mask;
-            for (int w = 0; w < nwalls; ++w) {
-                const int wg = I.wall_begin + w;
-                const unsigned int bit = 1u << w;
-                bool hit;
-                if (d.has_tri && (I.tri_mask & bit)) {
-                    // within R of the vertices' bounding box (the region the reference
-                    // searches, Mercury3D::computeWallForces with TriangleWall::isLocal)
-                    // and the face-plane test that opens TriangleWall::getDistanceAndNormal,
-                    // R with the instance's largest interaction distance; k_tri finishes
-                    // it and settles the history bits of these walls
-                    hit = false;
-                    if (near_tri) {
-                        const WallGeom& tg = d.wgeom[wg];
-                        const double R = ps.w + I.max_interaction_distance;
-                        hit = xs.x > tg.tlo[0] - R && xs.x < tg.thi[0] + R && xs.y > tg.tlo[1] - R &&
-                              xs.y < tg.thi[1] + R && xs.z > tg.tlo[2] - R && xs.z < tg.thi[2] + R &&
-                              fabs(dot(xs - row3(tg.tv[0]), row3(tg.tfn))) < R;
-                        if (hit) thit |= bit;
-                    }
-                } else {
-                    d.slotw[(size_t)w * d.ncap + s] = SLOT_NONE;
-                    if (far_still & bit) {
-                        hit = false;
-                    } else {
-                        const dem_wall& wall = d.walls[wg];
-                        const dem_species_pair& sp = d.species[I.species_offset + is.y * ns + wall.species];
-                        double dist;
-                        V3 nrm;
-                        hit = wall_distance(wall, d.wgeom + wg, xs, ps.w + sp.interaction_distance, dist, nrm);
-                        if (hit) whit |= bit;
-                    }
-                }
-                if (hit) {
-                    wnew |= bit;
-                } else if (first && (wa & bit) && !(I.wall_off_mask & bit)) {
-                    for (int q = 0; q < hist_stride(NCOMP); ++q) // with a triangle contact's creation key
-                        d.whist[nb][whist_at(d.ncap, NCOMP, s, w) + q] = d.whist[c][whist_at(d.ncap, NCOMP, s, w) + q];
-                    wnew |= bit;
-                }
-            }
-        }
-        d.wact[nb][s] = wnew;
+    const int top = d.item_cap - 1 - (int)atomicAdd(&d.ctl->n_carry, 1u);
+    if (top < 0) {
+        atomicOr(&d.ctl->status, 1u << DEM_ERR_CAPACITY);
+        return UIDX_NONE;
     }
-    // ---- compact the contacts of the block into the item list ----
-    const unsigned int hits[4] = {hit0, hit1, hit2, hit3};
-    int nh = __popc(whit) + (thit ? 1 : 0);
+    const double2* from = reinterpret_cast<const double2*>(d.pool[pc] + pool_at(NCOMP, from_idx));
+    double2* to = reinterpret_cast<double2*>(d.pool[pc ^ 1] + pool_at(NCOMP, top));
 #pragma unroll
-    for (int w = 0; w < 4; ++w) nh += __popc(hits[w]);
-    int total;
-    const int off = block_exclusive_scan(nh, warp_sums, total);
-    if (threadIdx.x == 0) block_base = total ? (int)atomicAdd(&ctl->n_items, (unsigned)total) : 0;
-    __syncthreads();
-    int q = block_base + off;
-    if (nh == 0) return;
-    if (q + nh > d.item_cap) {
-        atomicOr(&ctl->status, 1u << DEM_ERR_CAPACITY);
-        return;
-    }
-    int nh_seen = 0;
-#pragma unroll
-    for (int w = 0; w < 4; ++w) {
-        unsigned int b = hits[w];
-        // the entry's spring of the last evaluation, where it had one, goes into
-        // the item (its pool index; -1: a new contact), and its spring of this
-        // evaluation will sit at the item's own index
-        const unsigned int aw = b ? d.act[c][(size_t)w * d.ncap + s] : 0u;
-        while (b) {
-            const int k = w * 32 + __ffs(b) - 1;
-            b &= b - 1;
-            const size_t e = nbr_at(d.ncap, s, k);
-            const int t = (nh_seen < HIT_KEEP) ? kept_t[nh_seen][threadIdx.x] : d.nbr[l][e];
-            ++nh_seen;
-            const int prev = ((aw >> (k & 31)) & 1u) ? d.hidx[c][e] : -1;
-            d.items[q] = make_int4(s, k, t, prev);
-            d.slot[e] = q;
-            d.hidx[nb][e] = q;
-            ++q;
-        }
-    }
-    unsigned int b = whit;
-    while (b) {
+    for (int q = 0; q < hist_stride(NCOMP) / 2; ++q) to[q] = from[q];
+    return uidx_kept(top);
+}
+
+// The triangle walls (bits) particle s is near enough to for k_tri: the
+// bounding box and face-plane tests, with the reach widened to the instance's
+// largest interaction distance. The history rows of the others are carried
+// over the first time step (whist, wact).
+template <int NCOMP>
+__device__ __forceinline__ unsigned int near_triangles(const DevPtrs& d, const InstanceDev& I, int s, V3 x, double r,
+                                                       int hc, bool first)
+{
+    const double R = r + I.max_interaction_distance;
+    unsigned int hit = 0u, kept = 0u;
+    for (unsigned int b = d.wcand[s] & I.tri_mask; b; b &= b - 1) {
         const int w = __ffs(b) - 1;
-        b &= b - 1;
-        d.items[q] = make_int4(s, ITEM_WALL + w, -1, 0);
-        d.slotw[(size_t)w * d.ncap + s] = q;
-        ++q;
+        const WallGeom& tg = d.wgeom[I.wall_begin + w];
+        if (triangle_near(tg, x, R) && triangle_plane_near(tg, x, R)) hit |= 1u << w;
     }
-    if (thit) { // its net share is summed after the other walls' shares
-        d.items[q] = make_int4(s, ITEM_TRI, (int)thit, 0);
-        d.slott[s] = q;
-        d.tri_list[atomicAdd(&ctl->n_tri, 1u)] = q;
+    if (first)
+        for (unsigned int b = d.wact[hc][s] & I.tri_mask & ~hit; b; b &= b - 1) {
+            const int w = __ffs(b) - 1;
+            kept |= 1u << w;
+            for (int q = 0; q < hist_stride(NCOMP); ++q) // with the creation key
+                d.whist[hc ^ 1][whist_at(d.ncap, NCOMP, s, w) + q] = d.whist[hc][whist_at(d.ncap, NCOMP, s, w) + q];
+        }
+    d.wact[hc ^ 1][s] = kept; // k_tri adds the triangles it makes contacts with
+    if (!hit) d.slott[s] = -1;
+    return hit;
+}
+
+// The predicate of a wall or triangle unit (out of line: few units are walls,
+// and their geometry would cost the pair path its registers): bit 0 it
+// touches, bit 1 an old contact of it may outlive the first time step.
+template <int NCOMP>
+__device__ __noinline__ int wall_unit_touches(const DevPtrs& d, int j, int2 u, int c, int hc, bool first)
+{
+    const double4 ps = d.pr[c][u.x];
+    const int4 is = d.info[c][u.x];
+    const InstanceDev& I = d.inst[is.z];
+    if (u.y == UNIT_TRI) {
+        const unsigned int mask = near_triangles<NCOMP>(d, I, u.x, xyz(ps), ps.w, hc, first);
+        d.uidx[hc ^ 1][j] = (int)mask; // for k_tri's item (k_units reads it back)
+        return mask != 0u ? 1 : 0;
     }
+    const int w = ~u.y, wg = I.wall_begin + w;
+    if ((I.wall_off_mask >> w) & 1u) return 0;
+    const dem_wall& wall = d.walls[wg];
+    const dem_species_pair& sp = d.species[I.species_offset + is.y * I.n_species + wall.species];
+    double dist;
+    V3 nrm;
+    return wall_distance(wall, d.wgeom + wg, xyz(ps), ps.w + sp.interaction_distance, dist, nrm) ? 3 : 2;
+}
+
+// Outward normal (x, y, z) of a touching wall and the distance from it (w), out
+// of line for the same reason.
+__device__ __noinline__ double4 wall_normal_distance(const dem_wall* wall, const WallGeom* geom, double x, double y,
+                                                     double z, double R)
+{
+    double dist;
+    V3 nrm;
+    wall_distance(*wall, geom, v3(x, y, z), R, dist, nrm);
+    return make_double4(nrm.x, nrm.y, nrm.z, dist);
 }
 
 // RECORD: this launch may be the last force evaluation of a dem_step call,
@@ -396,144 +326,250 @@ __global__ void __launch_bounds__(BLOCK) k_detect(DevPtrs d)
 // MINB: resident blocks per SM the registers are budgeted for (4: 128
 // registers a thread; 5: 102; 6: 85; 3: 168), i.e. warps in flight against
 // spills; the time-step variant is compiled for 3 to 6 (dem_autotune).
+//
+// Bound by the latency of its gathers and of the laws' FP64 division and
+// square-root chains, not by DRAM. One flat list of owned pairs and walls
+// instead of a thread per particle walking its row: no divergence in the
+// predicate, UNITS_IN_FLIGHT gathers per thread, and neither an item list nor
+// per-entry marks pass through HBM between a detecting and an evaluating
+// kernel. A launch takes equal chunks: with few units every block gets one of
+// at least a warp, so a small system still spreads over all SMs.
 template <int MODE, int NLAW, int FLAW, int NCOMP, bool RECORD, int MINB = 4>
-__global__ void __launch_bounds__(CONTACT_BLOCK, MINB) k_contacts(DevPtrs d)
+__global__ void __launch_bounds__(UNIT_BLOCK, MINB) k_units(const __grid_constant__ DevPtrs d, int chunk_max)
 {
+    constexpr int UNITS_IN_FLIGHT = MINB <= 4 ? 4 : 2; // within the register budget
+    __shared__ TableStage tables;
+    __shared__ unsigned short hit_of[UNIT_CHUNK_MAX];
+    __shared__ int n_hit, item0;
     Control* ctl = d.ctl;
-    const int c = ctl->cur, nb = c ^ 1, pc = ctl->pcur;
+    const int c = ctl->cur, l = ctl->lbuf, hc = ctl->hcur, hn = hc ^ 1, pc = ctl->pcur;
     const bool final_step = (MODE == 0) ? true : (ctl->final_step != 0);
     const bool record = RECORD && final_step && ctl->record;
     const bool first = (MODE == 1) && ctl->first_step;
-    const int n_items = min((int)ctl->n_items, d.item_cap);
+    const int n_units = min(ctl->n_units, d.unit_cap);
     const double dt = d.dt;
-    __shared__ TableStage tables;
     stage_tables(d, tables);
+    if (threadIdx.x == 0) n_hit = 0;
     const dem_species_pair* species = staged_species(d, tables);
-    const int stride = gridDim.x * blockDim.x;
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    int4 next = q < n_items ? d.items[q] : make_int4(0, 0, 0, 0);
-    for (; q < n_items; q += stride) {
-        const int4 item = next; // the next item is read while this one is evaluated
-        if (q + stride < n_items) next = d.items[q + stride];
-        const int s = item.x, kq = item.y;
-        if (d.has_tri && kq == ITEM_TRI) continue; // k_tri
-        const double4 ps = d.pr[c][s];
-        const double4 vs = d.vm[c][s];
-        const double4 ws = d.wi[c][s];
-        const int4 is = d.info[c][s];
-        const InstanceDev& I = staged_inst(d, tables, is.z);
-        const int ns = I.n_species;
-        const V3 xq = xyz(ps), vq = xyz(vs), wq = xyz(ws);
-        const double rq = ps.w, mq = vs.w;
-        ContactGeom g;
-        Springs spr;
-        spr.slide = zero3(); spr.roll = zero3(); spr.tors = zero3();
-        const dem_species_pair* spp;
-        bool periodic = false, was_active = false;
-        int tq = 0, pid_i = 0;
-        const bool is_wall = kq >= ITEM_WALL;
-        double* hdst;
-        size_t hb;
-        V3 xt = zero3();
-        int rv = 0; // I's entry for this pair (reverse index), read with the other gathers
-        if (is_wall) {
-            // DPMBase::computeForcesDueToWalls / BaseWall::getInteractionWith
-            // (DPMBase.cc:3188-3215, BaseWall.cc:367-437)
-            const int wl = kq - ITEM_WALL;
-            const int wg = I.wall_begin + wl;
-            const dem_wall& wall = d.walls[wg];
-            spp = &species[I.species_offset + is.y * ns + wall.species];
-            double dist;
-            V3 nrm;
-            wall_distance(wall, d.wgeom + wg, xq, rq + spp->interaction_distance, dist, nrm);
-            g.n = -nrm;
-            g.distance = dist;
-            g.overlap = rq - dist;
-            g.c = xq - (rq - 0.5 * g.overlap) * g.n;
-            g.xp = xq; g.vp = vq; g.wp = wq; g.inv_mass_p = mq; g.curv_p = 1.0 / rq;
-            g.xi = v3(wall.position[0], wall.position[1], wall.position[2]);
-            g.vi = v3(wall.velocity[0], wall.velocity[1], wall.velocity[2]);
-            g.wi = v3(wall.angular_velocity[0], wall.angular_velocity[1], wall.angular_velocity[2]);
-            g.inv_mass_i = 0.0;
-            g.curv_i = 0.0;
-            g.i_is_wall = true;
-            hb = whist_at(d.ncap, NCOMP, s, wl);
-            hdst = d.whist[nb];
-            was_active = (d.wact[c][s] >> wl) & 1u;
-            if (was_active) load_springs(d.whist[c], hb, NCOMP, spr);
-            pid_i = wg;
-        } else {
-            const size_t e = nbr_at(d.ncap, s, kq);
-            tq = item.z;
-            rv = d.rev[e];
-            hb = pool_at(NCOMP, q); // this evaluation's spring sits at the item's index
-            // the spring of the last evaluation (item.w; -1 for a new contact, whose
-            // record 0 is read and not used): read before anything else needs it
-            Springs own;
-            load_springs(d.pool[pc], pool_at(NCOMP, max(item.w, 0)), NCOMP, own);
-            const double4 pt = d.pr[c][tq];
-            const int4 it = d.info[c][tq];
-            const double4 vt4 = d.vm[c][tq];
-            const double4 wt4 = d.wi[c][tq];
-            xt = image_of(I, xq, xyz(pt), periodic);
-            // this particle is P: the lower id, or the real particle against
-            // the partner's periodic ghost (DPMBase.cc:3129-3139)
-            const V3 branch = xq - xt;
-            const double d2 = len2(branch);
-            spp = &species[I.species_offset + is.y * ns + it.y];
-            g.distance = sqrt(d2);
-            g.n = branch / g.distance;
-            g.overlap = rq + pt.w - g.distance;
-            g.xp = xq; g.vp = vq; g.wp = wq; g.inv_mass_p = mq;
-            g.xi = xt; g.vi = xyz(vt4); g.wi = xyz(wt4); g.inv_mass_i = vt4.w;
-            g.c = g.xp - (rq - 0.5 * g.overlap) * g.n;
-            g.curv_p = 1.0 / rq;
-            g.curv_i = 1.0 / pt.w;
-            g.i_is_wall = false;
-            hdst = d.pool[pc ^ 1];
-            was_active = item.w >= 0;
-            // the higher-id side of a periodic pair restarts every step from the
-            // reversed spring of the lower-id side (InteractionHandler.cc:316-368,
-            // BaseInteraction::copySwitchPointer / reverseHistory)
-            const bool derived = periodic && (is.x > it.x);
-            if (derived) {
-                const int m = rv;
-                if ((d.act[c][(size_t)(m >> 5) * d.ncap + tq] >> (m & 31)) & 1u) {
-                    load_springs(d.pool[pc], pool_at(NCOMP, d.hidx[c][nbr_at(d.ncap, tq, m)]), NCOMP, spr);
+    const bool need_info = !d.single_instance || d.n_species_table > 1; // else instance 0, species 0
+    const double4* pr = d.pr[c];
+    const int4* info = d.info[c];
+    const int2* unit = d.unit[l];
+    // equal chunks of at most chunk_max units, a multiple of a warp each
+    const long long most = (long long)gridDim.x * chunk_max;
+    const long long passes = (n_units + most - 1) / most;
+    const int chunk = passes ? (int)(((n_units + passes * gridDim.x - 1) / (passes * gridDim.x) + 31) / 32) * 32 : 32;
+
+    for (unsigned int c0u = blockIdx.x * (unsigned int)chunk; c0u < (unsigned int)n_units;
+         c0u += gridDim.x * (unsigned int)chunk) {
+        const int c0 = (int)c0u;
+        const int m = min(chunk, n_units - c0);
+        // ---- the predicate ----
+        unsigned int hits = 0u, others = 0u; // bit i: unit c0 + threadIdx.x + i * UNIT_BLOCK touches / is no pair
+#pragma unroll 1
+        for (int i0 = 0; i0 * UNIT_BLOCK < m; i0 += UNITS_IN_FLIGHT) {
+            int2 un[UNITS_IN_FLIGHT];
+            double4 ps[UNITS_IN_FLIGHT], pt[UNITS_IN_FLIGHT];
+#pragma unroll
+            for (int i = 0; i < UNITS_IN_FLIGHT; ++i) {
+                const int k = threadIdx.x + (i0 + i) * UNIT_BLOCK;
+                un[i] = k < m ? unit[c0 + k] : make_int2(-1, -1);
+            }
+#pragma unroll
+            for (int i = 0; i < UNITS_IN_FLIGHT; ++i)
+                if (un[i].y >= 0) {
+                    ps[i] = pr[un[i].x];
+                    pt[i] = pr[un[i].y];
+                }
+#pragma unroll
+            for (int i = 0; i < UNITS_IN_FLIGHT; ++i) {
+                const int2 u = un[i];
+                if (u.y < 0) {
+                    if (u.x >= 0) others |= 1u << (i0 + i);
+                    continue;
+                }
+                double idist = 0.0; // x + 0.0 == x: skipping the lookup keeps the predicate exact
+                V3 xt = xyz(pt[i]);
+                bool periodic = false;
+                if (d.any_periodic || !d.zero_idist) {
+                    const InstanceDev& I = d.inst[d.single_instance ? 0 : info[u.x].z];
+                    if (!d.zero_idist)
+                        idist = d.species[I.species_offset + info[u.x].y * I.n_species + info[u.y].y].interaction_distance;
+                    xt = image_of(I, xyz(ps[i]), xt, periodic);
+                }
+                const double sum = pt[i].w + ps[i].w + idist; // rI + rP + distance (BaseParticle.cc:695-697)
+                bool hit = !(len2(xyz(ps[i]) - xt) >= sum * sum);
+                if (periodic && !hit) { // the partner's own view of a periodic pair
+                    const V3 xs = image_of(d.inst[d.single_instance ? 0 : info[u.x].z], xyz(pt[i]), xyz(ps[i]), periodic);
+                    hit = !(len2(xyz(pt[i]) - xs) >= sum * sum);
+                }
+                if (hit) {
+                    hits |= 1u << (i0 + i);
+                } else {
+                    const int j = c0 + threadIdx.x + (i0 + i) * UNIT_BLOCK;
+                    int v = UIDX_NONE;
+                    if (first) {
+                        const int from = uidx_spring(d.uidx[hc][j]);
+                        if (from >= 0) v = keep_spring<NCOMP>(d, pc, from);
+                    }
+                    d.uidx[hn][j] = v;
+                }
+            }
+        }
+        for (unsigned int b = others; b; b &= b - 1) {
+            const int i = __ffs(b) - 1, j = c0 + threadIdx.x + i * UNIT_BLOCK;
+            const int2 u = unit[j];
+            const int touch = wall_unit_touches<NCOMP>(d, j, u, c, hc, first);
+            if (touch & 1) {
+                hits |= 1u << i;
+            } else if (u.y != UNIT_TRI) {
+                int v = UIDX_NONE;
+                if (first && touch) {
+                    const int from = uidx_spring(d.uidx[hc][j]);
+                    if (from >= 0) v = keep_spring<NCOMP>(d, pc, from);
+                }
+                d.uidx[hn][j] = v;
+            }
+        }
+        // ---- the block's contacts ----
+        __syncthreads(); // n_hit is 0, the tables are staged, the last chunk's hit_of is read
+        for (unsigned int b = hits; b; b &= b - 1)
+            hit_of[atomicAdd(&n_hit, 1)] = (unsigned short)(threadIdx.x + (__ffs(b) - 1) * UNIT_BLOCK);
+        __syncthreads();
+        const int n_here = n_hit;
+        if (threadIdx.x == 0 && n_here) item0 = (int)atomicAdd(&ctl->n_items, (unsigned)n_here);
+        __syncthreads();
+        if (threadIdx.x == 0) n_hit = 0;
+        if (n_here && item0 + n_here > d.item_cap) {
+            if (threadIdx.x == 0) atomicOr(&ctl->status, 1u << DEM_ERR_CAPACITY);
+            for (int h = threadIdx.x; h < n_here; h += UNIT_BLOCK) {
+                const int j = c0 + hit_of[h];
+                d.uidx[hn][j] = UIDX_NONE;
+                if (unit[j].y == UNIT_TRI) d.slott[unit[j].x] = -1;
+            }
+            continue;
+        }
+        for (int h = threadIdx.x; h < n_here; h += UNIT_BLOCK) {
+            const int j = c0 + hit_of[h];
+            const int q = item0 + h;
+            const int2 u = unit[j];
+            if (d.has_tri && u.y == UNIT_TRI) { // its net share is summed after the other walls' shares
+                d.slott[u.x] = q;
+                d.tri_list[atomicAdd(&ctl->n_tri, 1u)] = make_int4(u.x, q, d.uidx[hn][j], 0);
+                continue;
+            }
+            const int from = uidx_spring(d.uidx[hc][j]);
+            d.uidx[hn][j] = q;
+            const bool is_wall = u.y < 0;
+            // view 0: P is u.x, the lower id (or a wall's particle); view 1, only of
+            // a periodic pair: P is the other real particle, against u.x's ghost
+#pragma unroll 1
+            for (int view = 0;; ++view) {
+                const int s = view ? u.y : u.x, t = view ? u.x : u.y;
+                // the spring of the last evaluation (record 0 is read and not used when
+                // there is none): read before anything else needs it
+                Springs spr;
+                load_springs(d.pool[pc], pool_at(NCOMP, max(from, 0)), NCOMP, spr);
+                const double4 ps = pr[s];
+                const double4 vs = d.vm[c][s];
+                const double4 ws = d.wi[c][s];
+                const int4 is = (need_info || record) ? info[s] : make_int4(0, 0, 0, 0);
+                const InstanceDev& I = staged_inst(d, tables, is.z);
+                const V3 xq = xyz(ps), vq = xyz(vs), wq = xyz(ws);
+                const double rq = ps.w, mq = vs.w;
+                ContactGeom g;
+                const dem_species_pair* spp;
+                bool periodic = false, touches = true;
+                int pid_i = 0;
+                V3 xt = zero3();
+                if (is_wall) {
+                    const int wg = I.wall_begin + ~t;
+                    const dem_wall& wall = d.walls[wg];
+                    spp = &species[I.species_offset + is.y * I.n_species + wall.species];
+                    // DPMBase::computeForcesDueToWalls / BaseWall::getInteractionWith
+                    // (DPMBase.cc:3188-3215, BaseWall.cc:367-437)
+                    const double4 nd = wall_normal_distance(&wall, d.wgeom + wg, xq.x, xq.y, xq.z,
+                                                            rq + spp->interaction_distance);
+                    g.n = -xyz(nd);
+                    g.distance = nd.w;
+                    g.overlap = rq - nd.w;
+                    g.c = xq - (rq - 0.5 * g.overlap) * g.n;
+                    g.xp = xq; g.vp = vq; g.wp = wq; g.inv_mass_p = mq; g.curv_p = 1.0 / rq;
+                    g.xi = v3(wall.position[0], wall.position[1], wall.position[2]);
+                    g.vi = v3(wall.velocity[0], wall.velocity[1], wall.velocity[2]);
+                    g.wi = v3(wall.angular_velocity[0], wall.angular_velocity[1], wall.angular_velocity[2]);
+                    g.inv_mass_i = 0.0;
+                    g.curv_i = 0.0;
+                    g.i_is_wall = true;
+                    pid_i = wg;
+                } else {
+                    const double4 pt = pr[t];
+                    const double4 vt4 = d.vm[c][t];
+                    const double4 wt4 = d.wi[c][t];
+                    const int4 it = (need_info || record) ? info[t] : make_int4(0, 0, 0, 0);
+                    xt = image_of(I, xq, xyz(pt), periodic);
+                    const V3 branch = xq - xt;
+                    const double d2 = len2(branch);
+                    spp = &species[I.species_offset + is.y * I.n_species + it.y];
+                    if (periodic) { // each view decides for itself
+                        const double sum = pt.w + ps.w + spp->interaction_distance;
+                        touches = !(d2 >= sum * sum);
+                    }
+                    g.distance = sqrt(d2);
+                    g.n = branch / g.distance;
+                    g.overlap = rq + pt.w - g.distance;
+                    g.xp = xq; g.vp = vq; g.wp = wq; g.inv_mass_p = mq;
+                    g.xi = xt; g.vi = xyz(vt4); g.wi = xyz(wt4); g.inv_mass_i = vt4.w;
+                    g.c = g.xp - (rq - 0.5 * g.overlap) * g.n;
+                    g.curv_p = 1.0 / rq;
+                    g.curv_i = 1.0 / pt.w;
+                    g.i_is_wall = false;
+                    pid_i = it.x;
+                }
+                if (from < 0) {
+                    spr.slide = zero3(); spr.roll = zero3(); spr.tors = zero3();
+                } else if (view) {
+                    // the higher-id side of a periodic pair restarts every step from the
+                    // reversed spring of the lower-id side (InteractionHandler.cc:316-368,
+                    // BaseInteraction::copySwitchPointer / reverseHistory)
                     spr.slide = -spr.slide; spr.roll = -spr.roll; spr.tors = -spr.tors;
                 }
-            } else if (was_active) {
-                spr = own;
+                ContactOut out;
+                evaluate_contact<NLAW, FLAW>(*spp, g, spr, dt, out);
+                // shares as 16-byte stores (96-byte items: every item and half is 16-byte aligned)
+                double2* sh = reinterpret_cast<double2*>(d.shares + (size_t)q * SHARE) + 3 * view;
+                V3 fp = out.force;
+                V3 tp = out.torque - cross(xq - g.c, out.force);
+                if (!touches) fp = tp = zero3();
+                sh[0] = make_double2(fp.x, fp.y);
+                sh[1] = make_double2(fp.z, tp.x);
+                sh[2] = make_double2(tp.y, tp.z);
+                if (view) break;
+                // step 0 keeps the lower-id side's old spring of a periodic pair that
+                // existed at the initial evaluation (equal stamps,
+                // InteractionHandler.cc:339-352); read again here instead of kept in
+                // registers. A view that does not touch keeps no spring, but for that step.
+                Springs kept = spr;
+                if (periodic && ((first && from >= 0) || !touches)) {
+                    kept.slide = zero3(); kept.roll = zero3(); kept.tors = zero3();
+                    if (first && from >= 0) load_springs(d.pool[pc], pool_at(NCOMP, from), NCOMP, kept);
+                }
+                store_springs(d.pool[pc ^ 1], pool_at(NCOMP, q), NCOMP, kept);
+                if (record && touches) {
+                    const double meff = 1.0 / (g.inv_mass_p + g.inv_mass_i);
+                    write_record(d, is.x, pid_i, is_wall ? 1 : 0, periodic ? 1 : 0, s, is_wall ? pid_i : t, g, out, kept,
+                                 spring_energy(*spp, kept, meff));
+                }
+                if (is_wall) break;
+                if (!periodic) { // I's share of an ordinary pair
+                    const V3 fi = -out.force;
+                    const V3 ti = -out.torque + cross(xt - g.c, out.force);
+                    sh[3] = make_double2(fi.x, fi.y);
+                    sh[4] = make_double2(fi.z, ti.x);
+                    sh[5] = make_double2(ti.y, ti.z);
+                    break;
+                }
             }
-            pid_i = it.x;
-        }
-        ContactOut out;
-        evaluate_contact<NLAW, FLAW>(*spp, g, spr, dt, out);
-        // step 0 keeps the lower-id side's old spring of a periodic pair that
-        // existed at the initial evaluation (equal stamps, InteractionHandler.cc:339-352);
-        // that side is not derived and was active, so its old spring is its own
-        // stored one, read again here instead of kept in registers
-        Springs kept = spr;
-        if (first && periodic && !(is.x > pid_i) && was_active) load_springs(d.pool[pc], pool_at(NCOMP, item.w), NCOMP, kept);
-        store_springs(hdst, hb, NCOMP, kept);
-        // shares as 16-byte stores (96-byte items: every item and half is 16-byte aligned)
-        double2* sh = reinterpret_cast<double2*>(d.shares + (size_t)q * SHARE);
-        const V3 tp = out.torque - cross(xq - g.c, out.force);
-        sh[0] = make_double2(out.force.x, out.force.y);
-        sh[1] = make_double2(out.force.z, tp.x);
-        sh[2] = make_double2(tp.y, tp.z);
-        if (!is_wall && !periodic) { // I's share of an ordinary pair, announced in I's own entry
-            const V3 fi = -out.force;
-            const V3 ti = -out.torque + cross(xt - g.c, out.force);
-            sh[3] = make_double2(fi.x, fi.y);
-            sh[4] = make_double2(fi.z, ti.x);
-            sh[5] = make_double2(ti.y, ti.z);
-            d.slot[nbr_at(d.ncap, tq, rv)] = SLOT_I_BASE - q;
-        }
-        if (record && (is_wall || !periodic || is.x < pid_i)) {
-            const double meff = 1.0 / (g.inv_mass_p + g.inv_mass_i);
-            write_record(d, is.x, pid_i, is_wall ? 1 : 0, periodic ? 1 : 0, s, is_wall ? pid_i : tq, g, out, kept,
-                         spring_energy(*spp, kept, meff));
         }
     }
 }
@@ -573,16 +609,15 @@ __global__ void __launch_bounds__(TRI_BLOCK) k_tri(DevPtrs d)
     constexpr int MAXT = DEM_MAX_TRIANGLE_CONTACTS;
     static_assert(NCOMP % 2 == 1, "the pad word of a history row holds the creation key");
     Control* ctl = d.ctl;
-    const int c = ctl->cur, nb = c ^ 1;
+    const int c = ctl->cur, hc = ctl->hcur, hn = hc ^ 1;
     const bool final_step = (MODE == 0) ? true : (ctl->final_step != 0);
     const bool record = final_step && ctl->record;
     const bool first = (MODE == 1) && ctl->first_step;
     const int n_tri = min((int)ctl->n_tri, d.n);
     const double dt = d.dt;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_tri; t += gridDim.x * blockDim.x) {
-        const int q = d.tri_list[t];
-        const int4 item = d.items[q];
-        const int s = item.x;
+        const int4 item = d.tri_list[t];
+        const int s = item.x, q = item.y;
         const unsigned int mask = (unsigned int)item.z;
         const double4 ps = d.pr[c][s];
         const double4 vs = d.vm[c][s];
@@ -592,7 +627,7 @@ __global__ void __launch_bounds__(TRI_BLOCK) k_tri(DevPtrs d)
         const int ns = I.n_species;
         const V3 xq = xyz(ps), vq = xyz(vs), wq = xyz(ws);
         const double rq = ps.w, mq = vs.w;
-        const unsigned int was = d.wact[c][s];
+        const unsigned int was = d.wact[hc][s];
         int ew[MAXT], esw[MAXT], ord[MAXT]; // ord: entries in interaction-list order
         double eov[MAXT], eel[MAXT], ek[MAXT];
         const double step_key = 16.0 * (double)ctl->steps_done;
@@ -667,8 +702,8 @@ __global__ void __launch_bounds__(TRI_BLOCK) k_tri(DevPtrs d)
                 es[k].slide = zero3(); es[k].roll = zero3(); es[k].tors = zero3();
                 if (!first && ((was >> w) & 1u)) { // the contact with this triangle from the last step
                     const size_t hb = whist_at(d.ncap, NCOMP, s, w);
-                    load_springs(d.whist[c], hb, NCOMP, es[k]);
-                    ek[k] = d.whist[c][hb + NCOMP];
+                    load_springs(d.whist[hc], hb, NCOMP, es[k]);
+                    ek[k] = d.whist[hc][hb + NCOMP];
                 } else {
                     ek[k] = step_key + (double)(made++);
                 }
@@ -719,7 +754,7 @@ __global__ void __launch_bounds__(TRI_BLOCK) k_tri(DevPtrs d)
         sh[2] = make_double2(T.y, T.z);
         // history: each triangle keeps the first contact (in order) now attached
         // to it; at the first step after the initial evaluation a contact of that
-        // evaluation that no entry took outlives the step (as k_detect carries them)
+        // evaluation that no entry took outlives the step (as near_triangles carries them)
         unsigned int kept_bits = 0u;
         for (int o = 0; o < ne; ++o) {
             const int e = ord[o];
@@ -727,10 +762,10 @@ __global__ void __launch_bounds__(TRI_BLOCK) k_tri(DevPtrs d)
             if (kept_bits & bit) continue;
             kept_bits |= bit;
             const size_t hb = whist_at(d.ncap, NCOMP, s, ew[e]);
-            store_springs(d.whist[nb], hb, NCOMP, es[e]);
-            d.whist[nb][hb + NCOMP] = ek[e];
+            store_springs(d.whist[hn], hb, NCOMP, es[e]);
+            d.whist[hn][hb + NCOMP] = ek[e];
         }
-        d.wact[nb][s] = (d.wact[nb][s] & ~mask) | kept_bits;
+        d.wact[hn][s] = (d.wact[hn][s] & ~mask) | kept_bits;
         if (MODE == 0) { // kept for the first time step
             double* rec = d.tri_first + (size_t)ci * MAXT * TRI_REC;
             for (int o = 0; o < ne; ++o, rec += TRI_REC) {
@@ -767,10 +802,11 @@ __global__ void __launch_bounds__(BLOCK, SUM_THREADS_PER_SM / BLOCK) k_sum(DevPt
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     Control* ctl = d.ctl;
-    const int c = ctl->cur, l = ctl->lbuf, nb = c ^ 1;
+    const int c = ctl->cur, to = c ^ ctl->spare;
+    const int* uidx = d.uidx[ctl->hcur ^ 1]; // of this evaluation
     const bool final_step = (MODE == 0) ? true : (ctl->final_step != 0);
     const double dt = d.dt;
-    if (s == 0) { // k_contacts and k_tri are done: the next evaluation starts new lists
+    if (s == 0) { // k_units and k_tri are done: the next evaluation starts new lists
         // the springs kept at the pool top in the first time step must not have
         // met this evaluation's items
         if (ctl->n_carry && (unsigned long long)ctl->n_items + ctl->n_carry > (unsigned long long)d.item_cap)
@@ -787,51 +823,57 @@ __global__ void __launch_bounds__(BLOCK, SUM_THREADS_PER_SM / BLOCK) k_sum(DevPt
         double4 qs = d.qo[c][s];
         const int4 is = d.info[c][s];
         const InstanceDev& I = d.inst[is.z];
+        const int u0 = d.ubase[s], u1 = d.wbase[s]; // its own pairs' units
+        const unsigned int walls = d.wcand[s];
         // ---- the shares in list order, the body force, the wall shares ----
         V3 F = zero3(), T = zero3();
-        const int count = min(d.cnt[l][s], d.cap);
-        constexpr int B = 4; // slots read together, then their shares
-        for (int k0 = 0; k0 < count; k0 += B) {
-            int qs_[B];
+        const int count = min(d.cnt[s], d.cap);
+        constexpr int E = 8, B = 4; // entries whose units, then items are read together; shares read together
+        for (int e0 = 0; e0 < count; e0 += E) {
+            int q[E];
 #pragma unroll
-            for (int j = 0; j < B; ++j) qs_[j] = (k0 + j < count) ? d.slot[nbr_at(d.ncap, s, k0 + j)] : SLOT_NONE;
-            double sh6[B][6];
+            for (int j = 0; j < E; ++j) q[j] = (e0 + j < count) ? d.epair[nbr_at(d.ncap, s, e0 + j)] : -1;
+            // a pair's units are its lower id's: the particle's own half is P's
+            // if the unit lies among its own units
+            unsigned int half = 0u;
 #pragma unroll
-            for (int j = 0; j < B; ++j) {
-                int q = qs_[j];
-                int half = 0;
-                if (q <= SLOT_I_BASE) {
-                    q = SLOT_I_BASE - q;
-                    half = 6;
-                }
-                if (q >= 0) {
-                    const double2* sh = reinterpret_cast<const double2*>(d.shares + (size_t)q * SHARE + half);
-                    const double2 a = sh[0], b = sh[1], e2 = sh[2];
-                    sh6[j][0] = a.x; sh6[j][1] = a.y; sh6[j][2] = b.x;
-                    sh6[j][3] = b.y; sh6[j][4] = e2.x; sh6[j][5] = e2.y;
-                }
+            for (int j = 0; j < E; ++j) {
+                if (q[j] < u0 || q[j] >= u1) half |= 1u << j;
+                if (q[j] >= 0) q[j] = uidx[q[j]];
             }
 #pragma unroll
-            for (int j = 0; j < B; ++j) // in list order
-                if (qs_[j] >= 0 || qs_[j] <= SLOT_I_BASE) {
-                    F += v3(sh6[j][0], sh6[j][1], sh6[j][2]);
-                    T += v3(sh6[j][3], sh6[j][4], sh6[j][5]);
-                }
+            for (int k0 = 0; k0 < E; k0 += B) {
+                double sh6[B][6];
+#pragma unroll
+                for (int j = 0; j < B; ++j)
+                    if (q[k0 + j] >= 0) {
+                        const double2* sh = reinterpret_cast<const double2*>(d.shares + (size_t)q[k0 + j] * SHARE) +
+                                            3 * ((half >> (k0 + j)) & 1u);
+                        const double2 a = sh[0], b = sh[1], e2 = sh[2];
+                        sh6[j][0] = a.x; sh6[j][1] = a.y; sh6[j][2] = b.x;
+                        sh6[j][3] = b.y; sh6[j][4] = e2.x; sh6[j][5] = e2.y;
+                    }
+#pragma unroll
+                for (int j = 0; j < B; ++j) // in list order
+                    if (q[k0 + j] >= 0) {
+                        F += v3(sh6[j][0], sh6[j][1], sh6[j][2]);
+                        T += v3(sh6[j][3], sh6[j][4], sh6[j][5]);
+                    }
+            }
         }
         if (!(is.w & FLAG_FIXED)) { // DPMBase::computeExternalForces (DPMBase.cc:3168-3179)
             const double m = 1.0 / vs.w;
             F += v3(I.gravity[0], I.gravity[1], I.gravity[2]) * m - d.drag * xyz(vs);
-            const int nw = I.wall_end - I.wall_begin;
-            for (int w = 0; w < nw; ++w) {
-                if (d.has_tri && ((I.tri_mask >> w) & 1u)) continue;
-                const int q = d.slotw[(size_t)w * d.ncap + s];
+            int u = u1;
+            for (unsigned int b = d.has_tri ? walls & ~I.tri_mask : walls; b; b &= b - 1, ++u) {
+                const int q = uidx[u];
                 if (q < 0) continue;
                 const double2* sh = reinterpret_cast<const double2*>(d.shares + (size_t)q * SHARE);
-                const double2 a = sh[0], b = sh[1], e2 = sh[2];
-                F += v3(a.x, a.y, b.x);
-                T += v3(b.y, e2.x, e2.y);
+                const double2 a = sh[0], b2 = sh[1], e2 = sh[2];
+                F += v3(a.x, a.y, b2.x);
+                T += v3(b2.y, e2.x, e2.y);
             }
-            if (d.has_tri && I.tri_mask) { // the net share of all triangle contacts (k_tri)
+            if (d.has_tri && (walls & I.tri_mask)) { // the net share of all triangle contacts (k_tri)
                 const int q = d.slott[s];
                 if (q >= 0) {
                     const double2* sh = reinterpret_cast<const double2*>(d.shares + (size_t)q * SHARE);
@@ -903,18 +945,19 @@ __global__ void __launch_bounds__(BLOCK, SUM_THREADS_PER_SM / BLOCK) k_sum(DevPt
             wn = make_double4(w.x, w.y, w.z, ws.w);
             qs = make_double4(q.q0, q.q1, q.q2, q.q3);
         }
-        int4 isn = is;
-        isn.w = wrapped ? (is.w | FLAG_WRAPPED) : (is.w & ~FLAG_WRAPPED);
-        if (MODE == 1 && !final_step && I.n_del && !(is.w & FLAG_DELETED) && deletion_check(I, xyz(pn))) {
-            park_deleted(ctl, pn, vn, wn, isn);
-            disp2 = 0.0;
+        if (MODE == 1) { // the initial evaluation leaves the state as it is
+            int4 isn = is;
+            isn.w = wrapped ? (is.w | FLAG_WRAPPED) : (is.w & ~FLAG_WRAPPED);
+            if (!final_step && I.n_del && !(is.w & FLAG_DELETED) && deletion_check(I, xyz(pn))) {
+                park_deleted(ctl, pn, vn, wn, isn);
+                disp2 = 0.0;
+            }
+            d.pr[to][s] = pn;
+            d.vm[to][s] = vn;
+            d.wi[to][s] = wn;
+            d.qo[to][s] = qs;
+            if (isn.w != is.w) d.info[to][s] = isn;
         }
-        d.pr[nb][s] = pn;
-        d.vm[nb][s] = vn;
-        d.wi[nb][s] = wn;
-        d.qo[nb][s] = qs;
-        d.info[nb][s] = isn;
-        d.caller[nb][s] = d.caller[c][s];
     }
     if (MODE == 1) { // maximum displacement of this step (for the skin test)
 #pragma unroll

@@ -14,10 +14,14 @@
 //   4 counting-sort scatter                                 (scatter_one)
 //   5 per-cell ordering by particle id, counters reset      (cell_sort_one)
 //   6 permutation gather of the state                       (gather_one)
-//   7 neighbour lists + contact-history carry-over          (build_one)
-//   8 reverse index of the new lists                        (rev_one)
+//   7 neighbour lists; each block takes the unit numbers of its
+//     particles from one counter                            (build_one)
+//   8 the units and, per list entry, its unit               (units_one)
+//   9 contact history of the old units to the new ones      (carry_one)
 //
-// and block 0 makes the new state buffer and lists current. This replaces
+// and block 0 makes the new state buffer and lists current. (The unit ranges
+// of different blocks follow each other in any order: no result depends on
+// a unit's number.) This replaces
 // the HGrid buckets and the InteractionHandler lookup of the reference
 // (Mercury3D.cc:224-416, InteractionHandler.cc:103-174).
 //
@@ -33,7 +37,7 @@
 namespace dem {
 
 constexpr int RB_BLOCK = 256;
-constexpr int RB_BARRIERS = 7;
+constexpr int RB_BARRIERS = 8;
 constexpr long long RB_POLL_LIMIT = 1ll << 24;
 
 __device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p)
@@ -117,7 +121,9 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
     if (!ctl->rebuild) return;
     __shared__ unsigned long long base_s;
     __shared__ int warp_sums[RB_BLOCK / 32];
-    const int hc = ctl->cur, lo = ctl->lbuf; // read by every block before the first barrier
+    // read by every block before the first barrier
+    const int hc = ctl->cur, lo = ctl->lbuf, hh = ctl->hcur;
+    const int old_units = min(ctl->n_units, d.unit_cap);
     if (threadIdx.x == 0) {
         const unsigned long long per = (unsigned long long)gridDim.x * RB_BARRIERS;
         base_s = ld_acquire_u64(barrier_ctr) / per * per;
@@ -125,6 +131,8 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
     __syncthreads();
     GridBarrier g{barrier_ctr, base_s, 0u};
     const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
+
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl->n_units_next = 0;
 
     // 1 keys and counts
     for (int i = gt; i < d.n; i += gs) keys_one(d, i, hc);
@@ -166,16 +174,38 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
     for (int s = gt; s < d.n; s += gs) gather_one(d, s, hc);
     if (!grid_barrier(g, ctl)) return;
 
-    // 7 lists and history carry-over
-    for (int s = gt; s < d.n; s += gs) build_one(d, s, hc, lo);
+    // 7 lists, then the block's range of unit numbers
+    __shared__ int unit_base;
+    for (int s0 = blockIdx.x * RB_BLOCK; s0 < d.n; s0 += gs) {
+        const int s = s0 + threadIdx.x;
+        int pairs = 0, walls = 0;
+        if (s < d.n) build_one(d, s, hc ^ 1, pairs, walls);
+        int total;
+        const int ex = block_exclusive_scan(pairs + walls, warp_sums, total);
+        if (threadIdx.x == 0) unit_base = atomicAdd(&ctl->n_units_next, total);
+        __syncthreads();
+        if (s < d.n) d.ubase[s] = unit_base + ex;
+    }
     if (!grid_barrier(g, ctl)) return;
 
-    // 8 reverse index of the new lists
-    for (int s = gt; s < d.n; s += gs) rev_one(d, s, lo ^ 1);
+    // 8 units of the new lists
+    for (int s = gt; s < d.n; s += gs) {
+        if (d.has_tri) carry_triangles(d, s, hh, hc);
+        units_one(d, s, lo ^ 1, hh ^ 1, hc ^ 1);
+    }
+    if (!grid_barrier(g, ctl)) return;
+
+    // 9 history
+    for (int j = gt; j < old_units; j += gs) carry_one(d, j, lo, hh, hc);
+    if (d.has_tri) // particles without a triangle unit have no history in the buffer written next either
+        for (int s = gt; s < d.n; s += gs)
+            if (!d.wact[hh ^ 1][s]) d.wact[hh][s] = 0u;
 
     if (blockIdx.x == 0 && threadIdx.x == 0) { // the gathered state and the new lists become current
         ctl->cur = hc ^ 1;
         ctl->lbuf = lo ^ 1;
+        ctl->hcur = hh ^ 1;
+        ctl->n_units = min(ctl->n_units_next, d.unit_cap);
         ctl->disp_acc = 0.0;
         ctl->n_rebuilds += 1;
     }

@@ -1,0 +1,63 @@
+"""The force evaluation's unit list (k_units): one thread per pair or wall
+candidate, chunks of whole warps per block, contacts compacted per block.
+
+Sizes where a chunk, a warp or a block is not full, from a lone pair to
+several blocks, against the oracle: contact pairs exact, per-contact forces
+bit-exact at the initial evaluation, and the first steps (in which springs of
+the initial evaluation may be kept without a contact) within the parity
+tests' tolerances. A list of one wall candidate and no pair, and none at all,
+run too; a run is bit-identical under every chunk size.
+"""
+import numpy as np
+import pytest
+
+import cases
+import harness as H
+from mercurydpm_fork_b200 import scenarios
+
+pytestmark = pytest.mark.gpu
+
+
+def _box(n, spacing=0.995):
+    nx = max(1, round(n ** (1 / 3)))
+    nz = -(-n // (nx * nx))
+    edge = lambda k: k * spacing * (1 + 1e-9)
+    return scenarios.settling_box(n=n, seed=n, box=(edge(nx), edge(nx), edge(nz)), spacing=spacing, jitter=0.004, vstd=0.05)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 11, 12, 43, 130, 1000, 2777])
+def test_sizes_around_warps_and_chunks(gpu, n):
+    sc = _box(n)
+    g, o = H.run_gpu(sc, 0), H.run_oracle(sc, 0)
+    assert H.pair_set(g["contacts"]) == H.pair_set(o["contacts"]) and len(o["contacts"]["id_p"]) > 0
+    np.testing.assert_array_equal(g["contacts"]["force"], o["contacts"]["force"])
+    np.testing.assert_array_equal(g["contacts"]["springs"], o["contacts"]["springs"])
+    for steps in (1, 2, 20):
+        g, o = H.run_gpu(sc, steps), H.run_oracle(sc, steps)
+        assert H.pair_set(g["contacts"]) == H.pair_set(o["contacts"])
+        assert H.rel_err(g["position"], o["position"], 1e-3) < 1e-13
+        for k in ("velocity", "force", "torque"):
+            assert H.rel_err(g[k], o[k]) < 1e-9, k
+        assert H.rel_err(g["contacts"]["springs"], o["contacts"]["springs"]) < 1e-9
+
+
+def test_no_unit_at_all(gpu):
+    sc = scenarios.settling_box(n=8, seed=1, box=(20, 20, 40), spacing=4.0)
+    g, o = H.run_gpu(sc, 5), H.run_oracle(sc, 5)
+    assert len(g["contacts"]["id_p"]) == 0
+    np.testing.assert_array_equal(g["position"], o["position"])
+
+
+@pytest.mark.parametrize("case", ["small_chute", "small_drum", "triangle_mesh"])
+def test_chunk_size_changes_nothing(gpu, case):
+    sc = getattr(cases, case)()
+    runs = []
+    for block in (64, 128, 256):
+        e = sc.engine()
+        e.set_tuning(detect_block=block, contacts_blocks_per_sm=3 if block == 256 else 5, sum_block=128)
+        e.step(30)
+        runs.append(dict(e.download(), springs=e.contacts()["springs"]))
+        e.close()
+    for other in runs[1:]:
+        for k in ("position", "velocity", "angular_velocity", "springs"):
+            np.testing.assert_array_equal(other[k], runs[0][k], err_msg=k)

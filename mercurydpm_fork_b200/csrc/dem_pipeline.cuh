@@ -309,14 +309,21 @@ __device__ __noinline__ int wall_unit_touches(const DevPtrs& d, int j, int2 u, i
     return wall_distance(wall, d.wgeom + wg, xyz(ps), ps.w + sp.interaction_distance, dist, nrm) ? 3 : 2;
 }
 
-// Outward normal (x, y, z) of a touching wall and the distance from it (w), out
-// of line for the same reason.
-__device__ __noinline__ double4 wall_normal_distance(const dem_wall* wall, const WallGeom* geom, double x, double y,
-                                                     double z, double R)
+// Outward normal (x, y, z) of the wall unit (s, ~w) touches and the distance
+// from it (w), out of line for the same reason, and called while little else is
+// live (DPMBase::computeForcesDueToWalls / BaseWall::getInteractionWith,
+// DPMBase.cc:3188-3215, BaseWall.cc:367-437).
+__device__ __noinline__ double4 wall_normal_distance(const DevPtrs& d, int c, int s, int w)
 {
+    const double4 ps = d.pr[c][s];
+    const int4 is = d.info[c][s];
+    const InstanceDev& I = d.inst[is.z];
+    const int wg = I.wall_begin + w;
+    const dem_wall& wall = d.walls[wg];
     double dist;
     V3 nrm;
-    wall_distance(*wall, geom, v3(x, y, z), R, dist, nrm);
+    wall_distance(wall, d.wgeom + wg, xyz(ps),
+                  ps.w + d.species[I.species_offset + is.y * I.n_species + wall.species].interaction_distance, dist, nrm);
     return make_double4(nrm.x, nrm.y, nrm.z, dist);
 }
 
@@ -337,7 +344,8 @@ __device__ __noinline__ double4 wall_normal_distance(const dem_wall* wall, const
 template <int MODE, int NLAW, int FLAW, int NCOMP, bool RECORD, int MINB = 4>
 __global__ void __launch_bounds__(UNIT_BLOCK, MINB) k_units(const __grid_constant__ DevPtrs d, int chunk_max)
 {
-    constexpr int UNITS_IN_FLIGHT = MINB <= 4 ? 4 : 2; // within the register budget
+    // more spills at these budgets (a step of the 1,000,000 drum: 290 us with 2, 301 us with 4)
+    constexpr int UNITS_IN_FLIGHT = 2;
     __shared__ TableStage tables;
     __shared__ unsigned short hit_of[UNIT_CHUNK_MAX];
     __shared__ int n_hit, item0;
@@ -466,6 +474,12 @@ __global__ void __launch_bounds__(UNIT_BLOCK, MINB) k_units(const __grid_constan
 #pragma unroll 1
             for (int view = 0;; ++view) {
                 const int s = view ? u.y : u.x, t = view ? u.x : u.y;
+                ContactGeom g;
+                if (is_wall) {
+                    const double4 nd = wall_normal_distance(d, c, s, ~t);
+                    g.n = -xyz(nd);
+                    g.distance = nd.w;
+                }
                 // the spring of the last evaluation (record 0 is read and not used when
                 // there is none): read before anything else needs it
                 Springs spr;
@@ -477,7 +491,6 @@ __global__ void __launch_bounds__(UNIT_BLOCK, MINB) k_units(const __grid_constan
                 const InstanceDev& I = staged_inst(d, tables, is.z);
                 const V3 xq = xyz(ps), vq = xyz(vs), wq = xyz(ws);
                 const double rq = ps.w, mq = vs.w;
-                ContactGeom g;
                 const dem_species_pair* spp;
                 bool periodic = false, touches = true;
                 int pid_i = 0;
@@ -486,13 +499,7 @@ __global__ void __launch_bounds__(UNIT_BLOCK, MINB) k_units(const __grid_constan
                     const int wg = I.wall_begin + ~t;
                     const dem_wall& wall = d.walls[wg];
                     spp = &species[I.species_offset + is.y * I.n_species + wall.species];
-                    // DPMBase::computeForcesDueToWalls / BaseWall::getInteractionWith
-                    // (DPMBase.cc:3188-3215, BaseWall.cc:367-437)
-                    const double4 nd = wall_normal_distance(&wall, d.wgeom + wg, xq.x, xq.y, xq.z,
-                                                            rq + spp->interaction_distance);
-                    g.n = -xyz(nd);
-                    g.distance = nd.w;
-                    g.overlap = rq - nd.w;
+                    g.overlap = rq - g.distance;
                     g.c = xq - (rq - 0.5 * g.overlap) * g.n;
                     g.xp = xq; g.vp = vq; g.wp = wq; g.inv_mass_p = mq; g.curv_p = 1.0 / rq;
                     g.xi = v3(wall.position[0], wall.position[1], wall.position[2]);
@@ -549,16 +556,15 @@ __global__ void __launch_bounds__(UNIT_BLOCK, MINB) k_units(const __grid_constan
                 // existed at the initial evaluation (equal stamps,
                 // InteractionHandler.cc:339-352); read again here instead of kept in
                 // registers. A view that does not touch keeps no spring, but for that step.
-                Springs kept = spr;
                 if (periodic && ((first && from >= 0) || !touches)) {
-                    kept.slide = zero3(); kept.roll = zero3(); kept.tors = zero3();
-                    if (first && from >= 0) load_springs(d.pool[pc], pool_at(NCOMP, from), NCOMP, kept);
+                    spr.slide = zero3(); spr.roll = zero3(); spr.tors = zero3();
+                    if (first && from >= 0) load_springs(d.pool[pc], pool_at(NCOMP, from), NCOMP, spr);
                 }
-                store_springs(d.pool[pc ^ 1], pool_at(NCOMP, q), NCOMP, kept);
+                store_springs(d.pool[pc ^ 1], pool_at(NCOMP, q), NCOMP, spr);
                 if (record && touches) {
                     const double meff = 1.0 / (g.inv_mass_p + g.inv_mass_i);
-                    write_record(d, is.x, pid_i, is_wall ? 1 : 0, periodic ? 1 : 0, s, is_wall ? pid_i : t, g, out, kept,
-                                 spring_energy(*spp, kept, meff));
+                    write_record(d, is.x, pid_i, is_wall ? 1 : 0, periodic ? 1 : 0, s, is_wall ? pid_i : t, g, out, spr,
+                                 spring_energy(*spp, spr, meff));
                 }
                 if (is_wall) break;
                 if (!periodic) { // I's share of an ordinary pair

@@ -18,7 +18,7 @@
 // (contact records arrive in launch order; the pair key makes their order
 // canonical). One warp per point then walks the bins that can reach it in
 // index order, each lane a fixed stride of every bin, and sums the lanes in a
-// fixed butterfly. The host divides by the volume of the averaged dimensions
+// fixed butterfly and divides by the volume of the averaged dimensions
 // (CG::volumeAverageVariables).
 // The contact records are those of the last force evaluation, i.e. the
 // interactions the reference holds when writeOutputFiles evaluates CG at the
@@ -26,7 +26,7 @@
 // meets across a periodic boundary the reference's kept interaction joins the
 // two real particles, InteractionHandler.cc:316-368, and CG uses those).
 #pragma once
-#include <cub/device/device_radix_sort.cuh>
+#include "dem_records.cuh"
 
 namespace dem {
 
@@ -322,7 +322,7 @@ constexpr int CG_ACC = 29;
 __global__ void __launch_bounds__(CG_GATHER) k_cg_gather(CGDev g, const CGParticle* prec, const int* porder,
                                                          const int* pstart, const int* pend, const CGContact* crec,
                                                          const int* corder, const int* cstart, const int* cend,
-                                                         int3 pw, int3 cw, double* out)
+                                                         int3 pw, int3 cw, double volume, double* out)
 {
     const int lane = threadIdx.x & 31;
     const int pt = blockIdx.x * (CG_GATHER / 32) + (threadIdx.x >> 5);
@@ -413,7 +413,7 @@ __global__ void __launch_bounds__(CG_GATHER) k_cg_gather(CGDev g, const CGPartic
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if (lane == f) mine = v;
     }
-    if (lane < CG_ACC) out[(size_t)pt * DEM_CG_NFIELDS + lane] = mine;
+    if (lane < CG_ACC) out[(size_t)pt * DEM_CG_NFIELDS + lane] = mine / volume;
 }
 
 } // namespace dem
@@ -479,12 +479,8 @@ extern "C" int dem_cg_eval(dem_handle* hh, const dem_cg_grid* grid, double* fiel
                                        (int*)nullptr, std::max(nrec, 1), 0, bits, h->stream));
     const size_t tmp_bytes = std::max(t1, std::max(t2, t3));
     // one scratch arena for the evaluation
-    size_t total = 0;
-    auto take = [&total](size_t bytes) {
-        const size_t at = total;
-        total += (bytes + 255) & ~(size_t)255;
-        return at;
-    };
+    Arena arena;
+    auto take = [&arena](size_t bytes) { return arena.take(bytes); };
     const size_t nn = std::max(n, 1), nr = std::max(nrec, 1);
     const size_t o_out = take(nvals * sizeof(double));
     const size_t o_prec = take(nn * sizeof(CGParticle));
@@ -495,9 +491,9 @@ extern "C" int dem_cg_eval(dem_handle* hh, const dem_cg_grid* grid, double* fiel
     const size_t o_bounds = take(4 * (size_t)npts * 4);
     const size_t o_wmax = take(6 * sizeof(int));
     const size_t o_tmp = take(tmp_bytes);
-    char* arena = nullptr;
-    CU(cudaMallocAsync((void**)&arena, total, h->stream));
-    auto at = [arena](size_t off) { return (void*)(arena + off); };
+    Scratch scratch(h);
+    CU(scratch.take(arena.total));
+    auto at = [&scratch](size_t off) { return (void*)(scratch.p + off); };
     double* dout = (double*)at(o_out);
     CGParticle* prec = (CGParticle*)at(o_prec);
     unsigned *pbin0 = (unsigned*)at(o_pbin0), *pbin1 = (unsigned*)at(o_pbin1);
@@ -535,11 +531,9 @@ extern "C" int dem_cg_eval(dem_handle* hh, const dem_cg_grid* grid, double* fiel
     CU(cudaStreamSynchronize(h->stream));
     k_cg_gather<<<(unsigned)((npts + CG_GATHER / 32 - 1) / (CG_GATHER / 32)), CG_GATHER, 0, h->stream>>>(g, prec, pslot1, pstart, pend, crec, cpos1, cstart, cend,
                                                             make_int3(w[0], w[1], w[2]), make_int3(w[3], w[4], w[5]),
-                                                            dout);
+                                                            volume, dout);
     CU(cudaGetLastError());
     CU(cudaMemcpyAsync(fields_out, dout, nvals * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaFreeAsync(arena, h->stream));
     CU(cudaStreamSynchronize(h->stream));
-    for (size_t k = 0; k < nvals; ++k) fields_out[k] /= volume;
     return DEM_OK;
 }

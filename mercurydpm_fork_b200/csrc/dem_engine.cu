@@ -18,6 +18,7 @@
 #include "dem_pipeline.cuh"
 #include "dem_rebuild.cuh"
 #include "dem_insert.cuh"
+#include "dem_records.cuh"
 
 using namespace dem;
 
@@ -70,6 +71,8 @@ struct Handle {
     dem_wall* d_walls = nullptr;
     WallGeom* d_wgeom = nullptr;
     double* d_stage = nullptr;         // caller-layout particle staging (18 words per slot)
+    char* d_scratch = nullptr;         // workspace kept between calls (Scratch), at most SCRATCH_KEEP bytes
+    size_t scratch_bytes = 0;
     double* d_batch = nullptr;         // per-instance balance rows of dem_reduce_batch
     std::vector<long long> layout;     // sizes the device arrays were allocated for
     Control* d_ctl = nullptr;
@@ -126,6 +129,57 @@ int dalloc(Handle* h, T** p, size_t count)
     *p = static_cast<T*>(ptr);
     return DEM_OK;
 }
+
+// Device workspace of one call, a single block. Up to SCRATCH_KEEP bytes it is
+// the handle's own, which grows and stays: the pool behind cudaMallocAsync gives
+// its memory back at every synchronisation, so that a block taken per call is
+// mapped anew each time (measured: 0.45 ms of a dem_reduce of 1,000 particles,
+// about 2 ms of a coarse-graining evaluation of 200,000). Larger needs (some
+// millions of contacts) are taken and given back per call. Calls on a handle are
+// serialised on its stream, so one block serves them all.
+constexpr size_t SCRATCH_KEEP = 512ull << 20;
+struct Scratch {
+    Handle* h;
+    char* p = nullptr;
+    bool own = false; // taken for this call
+    explicit Scratch(Handle* handle) : h(handle) {}
+    Scratch(const Scratch&) = delete;
+    Scratch& operator=(const Scratch&) = delete;
+    cudaError_t take(size_t bytes)
+    {
+        if (bytes > SCRATCH_KEEP) {
+            const cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, h->stream);
+            own = e == cudaSuccess;
+            return e;
+        }
+        if (bytes > h->scratch_bytes) {
+            if (h->d_scratch) cudaFree(h->d_scratch); // waits for the work that uses it
+            h->d_scratch = nullptr;
+            h->scratch_bytes = 0;
+            const size_t want = std::min(SCRATCH_KEEP, std::max<size_t>(bytes + bytes / 4, 1 << 16));
+            cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&h->d_scratch), want);
+            if (e != cudaSuccess) return e;
+            h->scratch_bytes = want;
+        }
+        p = h->d_scratch;
+        return cudaSuccess;
+    }
+    ~Scratch()
+    {
+        if (own) cudaFreeAsync(p, h->stream);
+    }
+};
+
+// offsets of the parts of one block, 256-byte aligned
+struct Arena {
+    size_t total = 0;
+    size_t take(size_t bytes)
+    {
+        const size_t at = total;
+        total += (bytes + 255) & ~(size_t)255;
+        return at;
+    }
+};
 
 void free_graphs(Handle* h)
 {
@@ -1592,19 +1646,14 @@ int dem_download_forces(dem_handle* hh, double* force, double* torque)
     int rc = read_control(h, &c);
     if (rc) return rc;
     const int n = h->d.n;
-    std::vector<double> f(3 * (size_t)n), t(3 * (size_t)n);
-    std::vector<int> caller(n);
-    CU(cudaMemcpyAsync(f.data(), h->d.force, f.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaMemcpyAsync(t.data(), h->d.torque, t.size() * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaMemcpyAsync(caller.data(), h->d.caller[c.cur], n * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+    if (n == 0) return DEM_OK;
+    const StagePtrs st = stage_ptrs(h->d_stage, (size_t)h->d.ncap);
+    k_unpack_forces<<<grid_for(n, 256), 256, 0, h->stream>>>(h->d, c.cur, st.pos, st.vel);
+    CU(cudaGetLastError());
+    const size_t bytes = 3 * (size_t)n * sizeof(double);
+    if (force) CU(cudaMemcpyAsync(force, st.pos, bytes, cudaMemcpyDeviceToHost, h->stream));
+    if (torque) CU(cudaMemcpyAsync(torque, st.vel, bytes, cudaMemcpyDeviceToHost, h->stream));
     CU(cudaStreamSynchronize(h->stream));
-    for (int s = 0; s < n; ++s) {
-        const int i = caller[s];
-        for (int k = 0; k < 3; ++k) {
-            if (force) force[3 * i + k] = f[3 * (size_t)s + k];
-            if (torque) torque[3 * i + k] = t[3 * (size_t)s + k];
-        }
-    }
     return DEM_OK;
 }
 
@@ -1624,27 +1673,63 @@ int dem_download_walls(dem_handle* hh, dem_wall* walls, int n)
     return DEM_OK;
 }
 
-// The contact records of the last evaluation in the order the contact
-// downloads report them: particle pairs first, then wall contacts, each by
-// (id of P, id of I or the caller's wall index).
-static int sorted_records(Handle* h, std::vector<ContactRecord>& rec)
+// The first m contact records of the last evaluation, in the order the contact
+// downloads report them (dem_records.cuh), into the host arrays of `to` (null: not
+// asked for).
+static int download_records(Handle* h, int64_t m, const RecordArrays& to)
+{
+    const unsigned nr = h->n_records;
+    if (m <= 0) return DEM_OK;
+    CU(cudaSetDevice(h->device));
+    size_t t1 = 0, t2 = 0;
+    CU(cub::DeviceRadixSort::SortPairs(nullptr, t1, (const unsigned*)nullptr, (unsigned*)nullptr, (const int*)nullptr,
+                                       (int*)nullptr, (int)nr, 0, 32, h->stream));
+    CU(cub::DeviceRadixSort::SortPairs(nullptr, t2, (const unsigned long long*)nullptr, (unsigned long long*)nullptr,
+                                       (const int*)nullptr, (int*)nullptr, (int)nr, 0, 33, h->stream));
+    Arena a;
+    const size_t n = nr;
+    const size_t o_key0 = a.take(n * 8), o_key1 = a.take(n * 8), o_idx0 = a.take(n * 4), o_idx1 = a.take(n * 4);
+    const size_t o_walls = a.take(std::max<size_t>(1, h->wall_caller.size()) * 4);
+    const size_t o_tmp = a.take(std::max(t1, t2));
+    struct Out {
+        void* host;
+        size_t width, at;
+    } out[10] = {{to.id_p, 4, 0}, {to.id_i, 4, 0}, {to.is_wall, 4, 0}, {to.periodic, 4, 0}, {to.springs, 72, 0},
+                 {to.force, 24, 0}, {to.overlap, 8, 0}, {to.contact_point, 24, 0}, {to.normal, 24, 0},
+                 {to.tangential, 24, 0}};
+    for (Out& o : out)
+        if (o.host) o.at = a.take(n * o.width);
+    Scratch scratch(h);
+    CU(scratch.take(a.total));
+    auto at = [&](size_t off) { return (void*)(scratch.p + off); };
+    auto dev = [&](const Out& o) { return o.host ? at(o.at) : nullptr; };
+    unsigned *k0 = (unsigned*)at(o_key0), *k1 = (unsigned*)at(o_key1);
+    int *i0 = (int*)at(o_idx0), *i1 = (int*)at(o_idx1), *walls = (int*)at(o_walls);
+    if (!h->wall_caller.empty())
+        CU(cudaMemcpyAsync(walls, h->wall_caller.data(), h->wall_caller.size() * 4, cudaMemcpyHostToDevice, h->stream));
+    k_record_keys_i<<<grid_for(nr, 256), 256, 0, h->stream>>>(h->d_records, nr, walls, k0, i0);
+    CU(cub::DeviceRadixSort::SortPairs(at(o_tmp), t1, k0, k1, i0, i1, (int)nr, 0, 32, h->stream));
+    k_record_keys_p<<<grid_for(nr, 256), 256, 0, h->stream>>>(h->d_records, nr, i1, (unsigned long long*)at(o_key0));
+    CU(cub::DeviceRadixSort::SortPairs(at(o_tmp), t2, (const unsigned long long*)at(o_key0),
+                                       (unsigned long long*)at(o_key1), i1, i0, (int)nr, 0, 33, h->stream));
+    const RecordArrays da{(int*)dev(out[0]), (int*)dev(out[1]), (int*)dev(out[2]), (int*)dev(out[3]), (double*)dev(out[4]),
+                          (double*)dev(out[5]), (double*)dev(out[6]), (double*)dev(out[7]), (double*)dev(out[8]),
+                          (double*)dev(out[9])};
+    k_record_arrays<<<grid_for(nr, 256), 256, 0, h->stream>>>(h->d_records, nr, i0, walls, da);
+    CU(cudaGetLastError());
+    for (const Out& o : out)
+        if (o.host) CU(cudaMemcpyAsync(o.host, at(o.at), (size_t)m * o.width, cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaStreamSynchronize(h->stream));
+    return DEM_OK;
+}
+
+// whether the contact records of the last evaluation can be read
+static int records_ready(Handle* h)
 {
     if (!h->uploaded || h->initial_pending) return fail(h, DEM_ERR_STATE, "no force evaluation yet (call dem_step)");
     if (!h->records_valid)
         return fail(h, DEM_ERR_CAPACITY, "contact records of the last evaluation overflowed; the buffer has grown, "
                                          "the next dem_step records all contacts");
-    CU(cudaSetDevice(h->device));
-    const unsigned nr = h->n_records;
-    rec.resize(nr);
-    if (nr) CU(cudaMemcpyAsync(rec.data(), h->d_records, nr * sizeof(ContactRecord), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaStreamSynchronize(h->stream));
-    for (auto& x : rec)
-        if (x.is_wall) x.id_i = h->wall_caller[x.id_i]; // report the caller's wall index
-    std::sort(rec.begin(), rec.end(), [](const ContactRecord& a, const ContactRecord& b) {
-        if (a.is_wall != b.is_wall) return a.is_wall < b.is_wall;
-        if (a.id_p != b.id_p) return a.id_p < b.id_p;
-        return a.id_i < b.id_i;
-    });
     return DEM_OK;
 }
 
@@ -1653,43 +1738,30 @@ int dem_download_contact_geometry(dem_handle* hh, double* contact_point, double*
 {
     Handle* h = reinterpret_cast<Handle*>(hh);
     if (!h || !count || capacity < 0) return fail(h, DEM_ERR_BAD_INPUT, "dem_download_contact_geometry: bad arguments");
-    std::vector<ContactRecord> rec;
-    int rc = sorted_records(h, rec);
+    int rc = records_ready(h);
     if (rc) return rc;
-    *count = (int64_t)rec.size();
-    const int64_t m = std::min<int64_t>(capacity, (int64_t)rec.size());
-    for (int64_t r = 0; r < m; ++r)
-        for (int k = 0; k < 3; ++k) {
-            if (contact_point) contact_point[3 * r + k] = rec[r].contact_point[k];
-            if (normal) normal[3 * r + k] = rec[r].normal[k];
-            if (tangential_force) tangential_force[3 * r + k] = rec[r].tangential[k];
-        }
-    return DEM_OK;
+    *count = (int64_t)h->n_records;
+    RecordArrays to{};
+    to.contact_point = contact_point;
+    to.normal = normal;
+    to.tangential = tangential_force;
+    if (!contact_point && !normal && !tangential_force) return DEM_OK;
+    return download_records(h, std::min<int64_t>(capacity, (int64_t)h->n_records), to);
 }
 
 int dem_download_contacts(dem_handle* hh, dem_contacts_soa* cs, int64_t capacity, int64_t* count)
 {
     Handle* h = reinterpret_cast<Handle*>(hh);
     if (!h || !count || capacity < 0) return fail(h, DEM_ERR_BAD_INPUT, "dem_download_contacts: bad arguments");
-    std::vector<ContactRecord> rec;
-    int rc = sorted_records(h, rec);
+    int rc = records_ready(h);
     if (rc) return rc;
-    const unsigned nr = (unsigned)rec.size();
-    *count = nr;
+    *count = (int64_t)h->n_records;
     if (!cs) return DEM_OK;
-    const int64_t m = std::min<int64_t>(capacity, nr);
-    for (int64_t r = 0; r < m; ++r) {
-        const ContactRecord& x = rec[r];
-        if (cs->id_p) cs->id_p[r] = x.id_p;
-        if (cs->id_i) cs->id_i[r] = x.id_i;
-        if (cs->is_wall) cs->is_wall[r] = x.is_wall;
-        if (cs->periodic) cs->periodic[r] = x.periodic;
-        if (cs->overlap) cs->overlap[r] = x.overlap;
-        for (int k = 0; k < 3; ++k)
-            if (cs->force) cs->force[3 * r + k] = x.force[k];
-        for (int k = 0; k < 9; ++k)
-            if (cs->springs) cs->springs[9 * r + k] = x.springs[k];
-    }
+    const int64_t m = std::min<int64_t>(capacity, (int64_t)h->n_records);
+    RecordArrays to{};
+    to.id_p = cs->id_p; to.id_i = cs->id_i; to.is_wall = cs->is_wall; to.periodic = cs->periodic;
+    to.springs = cs->springs; to.force = cs->force; to.overlap = cs->overlap;
+    if ((rc = download_records(h, m, to))) return rc;
     cs->n = m;
     return DEM_OK;
 }
@@ -1706,14 +1778,14 @@ int dem_reduce(dem_handle* hh, int instance, dem_globals* out)
     const unsigned nb = grid_for(n, 256);
     const unsigned nr = h->records_valid && !h->initial_pending ? h->n_records : 0;
     const unsigned nbr = grid_for(nr, 256);
-    double* dpart = nullptr;
     const size_t slots = (size_t)nb * RED_SLOTS + (size_t)nbr * 3;
-    CU(cudaMallocAsync((void**)&dpart, slots * sizeof(double), h->stream));
+    Scratch scratch(h);
+    CU(scratch.take(slots * sizeof(double)));
+    double* dpart = reinterpret_cast<double*>(scratch.p);
     k_reduce_particles<<<nb, 256, 0, h->stream>>>(h->d, instance, dpart);
     if (nr) k_reduce_records<<<nbr, 256, 0, h->stream>>>(h->d, instance, nr, dpart + (size_t)nb * RED_SLOTS);
     std::vector<double> part(slots);
     CU(cudaMemcpyAsync(part.data(), dpart, slots * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CU(cudaFreeAsync(dpart, h->stream));
     CU(cudaStreamSynchronize(h->stream));
     double acc[RED_SLOTS] = {0};
     for (unsigned b = 0; b < nb; ++b)
@@ -1905,19 +1977,18 @@ int dem_get_counts(dem_handle* hh, int64_t* list_entries, int64_t* contacts, int
     if (!h) return DEM_ERR_BAD_INPUT;
     if (!h->uploaded || h->initial_pending) return fail(h, DEM_ERR_STATE, "no force evaluation yet (call dem_step)");
     CU(cudaSetDevice(h->device));
-    Control c;
-    int rc = read_control(h, &c);
-    if (rc) return rc;
-    std::vector<int> cnt(h->d.n);
-    CU(cudaMemcpyAsync(cnt.data(), h->d.cnt, cnt.size() * sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    std::vector<ContactRecord> rec(h->records_valid ? h->n_records : 0);
-    if (!rec.empty())
-        CU(cudaMemcpyAsync(rec.data(), h->d_records, rec.size() * sizeof(ContactRecord), cudaMemcpyDeviceToHost,
-                           h->stream));
+    unsigned long long v[3] = {0, 0, 0};
+    const unsigned nr = h->records_valid ? h->n_records : 0;
+    Scratch scratch(h);
+    CU(scratch.take(sizeof(v)));
+    unsigned long long* dv = reinterpret_cast<unsigned long long*>(scratch.p);
+    CU(cudaMemsetAsync(dv, 0, sizeof(v), h->stream));
+    const long long most = std::max<long long>(h->d.n, nr);
+    k_count<<<(unsigned)std::min<long long>(grid_for(most, 256), 4ll * h->sm_count), 256, 0, h->stream>>>(h->d, nr, dv);
+    CU(cudaGetLastError());
+    CU(cudaMemcpyAsync(v, dv, sizeof(v), cudaMemcpyDeviceToHost, h->stream));
     CU(cudaStreamSynchronize(h->stream));
-    long long e = 0, pc = 0, wc = 0;
-    for (int v : cnt) e += v;
-    for (const auto& r : rec) (r.is_wall ? wc : pc) += 1;
+    const long long e = (long long)v[0], pc = (long long)v[1], wc = (long long)v[2];
     if (list_entries) *list_entries = e;
     if (contacts) *contacts = pc;
     if (wall_contacts) *wall_contacts = wc;
@@ -2107,6 +2178,7 @@ void dem_destroy(dem_handle* hh)
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     free_particle_arrays(h);
+    if (h->d_scratch) cudaFree(h->d_scratch);
     if (h->d_rtmp) cudaFree(h->d_rtmp);
     if (h->d_rstats) cudaFree(h->d_rstats);
     if (h->ev0) cudaEventDestroy(h->ev0);

@@ -16,6 +16,7 @@
 #include <cstring>
 #include <random>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/dem_surrogate.h"
@@ -41,6 +42,7 @@ struct Mlp {
     int capacity = 0;
     cudaStream_t stream = nullptr;
     std::string err;
+    char* block = nullptr;                                          // holds every array below
     unsigned* d_error = nullptr;
     float *p = nullptr, *g = nullptr, *m = nullptr, *v = nullptr; // params, grads, Adam moments (FP32)
     __nv_bfloat16* wb = nullptr;                                    // BF16 copy of the whole vector
@@ -53,7 +55,8 @@ struct Mlp {
     float *z1 = nullptr, *z2 = nullptr, *z3 = nullptr, *y = nullptr;
     __nv_bfloat16 *h1 = nullptr, *h2 = nullptr, *h3 = nullptr;
     __nv_bfloat16 *dyb = nullptr, *dz1 = nullptr, *dz2 = nullptr, *dz3 = nullptr;
-    float* loss = nullptr;
+    float *loss = nullptr, *loss_part = nullptr;
+    float* partial = nullptr;                                       // weight-gradient slices, MAX_SLICES parameter vectors
 };
 
 int fail(Mlp* h, int code, const std::string& msg)
@@ -95,15 +98,17 @@ __global__ void k_denorm_outputs(const float* y, const float* norm, int n, float
     out[i] = y[i] * norm[2 * NI + NO + c] + norm[2 * NI + c];
 }
 
-// loss = mean (y - t')^2 with t' the normalised target; dy = 2 (y - t') / (3 n)
-// in BF16. One block, rows in a fixed order.
-__global__ void __launch_bounds__(256) k_loss(const float* y, const float* t, const float* norm, int n,
-                                              __nv_bfloat16* dyb, float* loss)
+// dy = 2 (y - t') / (3 n) in BF16 with t' the normalised target, and each
+// block's part of the sum of (y - t')^2, its elements in a fixed order
+// (k_reduce_params adds the parts).
+constexpr int LOSS_BLOCK = 256;
+__global__ void __launch_bounds__(LOSS_BLOCK) k_loss(const float* y, const float* t, const float* norm, int n,
+                                                     __nv_bfloat16* dyb, float* part)
 {
-    __shared__ float sh[256];
+    __shared__ float sh[LOSS_BLOCK];
     float acc = 0.f;
     const float scale = 2.0f / (3.0f * (float)n);
-    for (int i = threadIdx.x; i < n * NO; i += blockDim.x) {
+    for (int i = blockIdx.x * LOSS_BLOCK + threadIdx.x; i < n * NO; i += gridDim.x * LOSS_BLOCK) {
         const int c = i % NO;
         const float tn = (t[i] - norm[2 * NI + c]) / norm[2 * NI + NO + c];
         const float d = y[i] - tn;
@@ -112,21 +117,11 @@ __global__ void __launch_bounds__(256) k_loss(const float* y, const float* t, co
     }
     sh[threadIdx.x] = acc;
     __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
+    for (int s = LOSS_BLOCK / 2; s > 0; s >>= 1) {
         if (threadIdx.x < s) sh[threadIdx.x] += sh[threadIdx.x + s];
         __syncthreads();
     }
-    if (threadIdx.x == 0) *loss = sh[0] / (3.0f * (float)n);
-}
-
-// bias gradient: column sums of a [n][cols] BF16 matrix
-__global__ void k_colsum(const __nv_bfloat16* d, int n, int cols, float* out)
-{
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
-    float s = 0.f;
-    for (int r = 0; r < n; ++r) s += __bfloat162float(d[(long long)r * cols + c]);
-    out[c] = s;
+    if (threadIdx.x == 0) part[blockIdx.x] = sh[0];
 }
 
 __global__ void k_to_bf16(const float* p, long long n, __nv_bfloat16* out)
@@ -135,13 +130,26 @@ __global__ void k_to_bf16(const float* p, long long n, __nv_bfloat16* out)
     if (i < n) out[i] = __float2bfloat16_rn(p[i]);
 }
 
-// Adam (Kingma and Ba 2015) with bias correction; refreshes the BF16 copy
-__global__ void k_adam(float* p, const float* g, float* m, float* v, long long n, float lr, float bc1, float bc2,
-                       __nv_bfloat16* wb)
+// The gradient of parameter i from the slices' partial sums in slice order, the
+// loss from the blocks' parts, and (step) Adam (Kingma and Ba 2015) with bias
+// correction, which refreshes the BF16 copy.
+__global__ void __launch_bounds__(256) k_reduce_params(const float* partial, int slices, long long stride, const float* loss_part,
+                                                       int loss_blocks, float loss_scale, float* loss, float* g, bool step,
+                                                       float* p, float* m, float* v, float lr, float bc1, float bc2,
+                                                       __nv_bfloat16* wb)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
+    if (i == 0) {
+        float s = 0.f;
+        for (int b = 0; b < loss_blocks; ++b) s += loss_part[b];
+        *loss = s / loss_scale;
+    }
+    if (i >= NPARAM) return;
+    float gi = 0.f;
+#pragma unroll 8
+    for (int s = 0; s < slices; ++s) gi += partial[(long long)s * stride + i];
+    g[i] = gi;
+    if (!step) return;
     const float mi = 0.9f * m[i] + 0.1f * gi;
     const float vi = 0.999f * v[i] + 0.001f * gi * gi;
     m[i] = mi;
@@ -152,30 +160,40 @@ __global__ void k_adam(float* p, const float* g, float* m, float* v, long long n
 }
 
 template <int BN>
-int launch_gemm(Mlp* h, GemmArgs a)
+int launch_layer(Mlp* h, GemmArgs a)
 {
-    using L = GemmSmem<BN>;
     static bool configured[64] = {false};
     if (!configured[h->device & 63]) {
-        CK(cudaFuncSetAttribute(k_gemm_bf16<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::BYTES));
+        CK(cudaFuncSetAttribute(k_layer<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, LayerSmem<BN>::bytes(LAYER_MAX_K)));
         configured[h->device & 63] = true;
     }
     a.error = h->d_error;
     const dim3 grid(grid1(a.M, GEMM_BM), grid1(a.N, BN));
-    k_gemm_bf16<BN><<<grid, GEMM_THREADS, L::BYTES, h->stream>>>(a);
+    k_layer<BN><<<grid, GEMM_THREADS, LayerSmem<BN>::bytes(a.K), h->stream>>>(a);
     CK(cudaGetLastError());
     return DEM_MLP_OK;
 }
 
-// C = A . B^T with the operand strides of GemmArgs; N <= 16 uses 16-wide tiles
+// C = A . B^T with the operand strides of GemmArgs, K <= 256; N <= 16 uses 16-wide tiles
 int gemm(Mlp* h, const __nv_bfloat16* A, long long a_sm, long long a_sk, const __nv_bfloat16* B, long long b_sn,
          long long b_sk, int M, int N, int K, int epi, const float* bias, const float* aux, float* out_f32,
          __nv_bfloat16* out_bf16, int ldc)
 {
     GemmArgs a{A, B, a_sm, a_sk, b_sn, b_sk, M, N, K, epi, bias, aux, out_f32, out_bf16, ldc, nullptr};
-    if (N <= 16) return launch_gemm<16>(h, a);
-    return launch_gemm<256>(h, a);
+    if (N <= 16) return launch_layer<16>(h, a);
+    return launch_layer<LAYER_BN>(h, a);
 }
+
+// Slices of the batch in the weight gradients: 64 samples each up to
+// MAX_SLICES of them (a batch of 1,024), longer ones beyond.
+constexpr int MAX_SLICES = 16;
+int slice_length(int n)
+{
+    const int chunks = (n + GEMM_BK - 1) / GEMM_BK;
+    return GEMM_BK * ((chunks + MAX_SLICES - 1) / MAX_SLICES);
+}
+constexpr int MAX_LOSS_BLOCKS = 64;
+constexpr long long PARAM_STRIDE = (NPARAM + 3) / 4 * 4; // of a slice: 16-byte rows
 
 } // namespace
 
@@ -203,55 +221,66 @@ int forward_fused(Mlp* h, int n)
     return DEM_MLP_OK;
 }
 
-// keep_z: store the pre-activations for a backward pass (training, one GEMM
-// per layer); without, the fused inference kernel
-int forward(Mlp* h, int n, bool keep_z = true)
+// the training pass: one product per layer, the pre-activations kept
+int forward(Mlp* h, int n)
 {
-    if (!keep_z) return forward_fused(h, n);
-    const int epi = keep_z ? EPI_BIAS_GELU : EPI_BIAS_GELU_H;
     int rc;
     const __nv_bfloat16* W = h->wb;
     const float* P = h->p;
     k_norm_inputs<<<grid1((long long)n * NI, 256), 256, 0, h->stream>>>(h->x, h->d_norm, n, h->xb);
     // z1 = x W1^T + b1, h1 = gelu(z1), ... (A rows = samples, B rows = output features)
-    if ((rc = gemm(h, h->xb, NI, 1, W + OFF_W1, NI, 1, n, NH, NI, epi, P + OFF_B1, nullptr, h->z1, h->h1, NH)))
+    if ((rc = gemm(h, h->xb, NI, 1, W + OFF_W1, NI, 1, n, NH, NI, EPI_BIAS_GELU, P + OFF_B1, nullptr, h->z1, h->h1, NH)))
         return rc;
-    if ((rc = gemm(h, h->h1, NH, 1, W + OFF_W2, NH, 1, n, NH, NH, epi, P + OFF_B2, nullptr, h->z2, h->h2, NH)))
+    if ((rc = gemm(h, h->h1, NH, 1, W + OFF_W2, NH, 1, n, NH, NH, EPI_BIAS_GELU, P + OFF_B2, nullptr, h->z2, h->h2, NH)))
         return rc;
-    if ((rc = gemm(h, h->h2, NH, 1, W + OFF_W3, NH, 1, n, NH, NH, epi, P + OFF_B3, nullptr, h->z3, h->h3, NH)))
+    if ((rc = gemm(h, h->h2, NH, 1, W + OFF_W3, NH, 1, n, NH, NH, EPI_BIAS_GELU, P + OFF_B3, nullptr, h->z3, h->h3, NH)))
         return rc;
     return gemm(h, h->h3, NH, 1, W + OFF_W4, NH, 1, n, NO, NH, EPI_BIAS_F32, P + OFF_B4, nullptr, h->y, nullptr, NO);
 }
 
-// gradient of the mean squared error into h->g; loss into h->loss
-int backward(Mlp* h, int n)
+// Gradient of the mean squared error into h->g, loss into h->loss; lr > 0: and
+// the Adam step (bias corrections bc1, bc2).
+int backward(Mlp* h, int n, float lr = 0.f, float bc1 = 1.f, float bc2 = 1.f)
 {
     int rc;
     const __nv_bfloat16* W = h->wb;
-    float* G = h->g;
-    k_loss<<<1, 256, 0, h->stream>>>(h->y, h->t, h->d_norm, n, h->dyb, h->loss);
-    // layer 4: dW4[o][i] = sum_b dy[b][o] h3[b][i]; db4 = colsum(dy); dz3 = (dy W4) gelu'(z3)
-    if ((rc = gemm(h, h->dyb, 1, NO, h->h3, 1, NH, NO, NH, n, EPI_STORE_F32, nullptr, nullptr, G + OFF_W4, nullptr, NH)))
-        return rc;
-    k_colsum<<<1, 32, 0, h->stream>>>(h->dyb, n, NO, G + OFF_B4);
+    const int loss_blocks = std::min(MAX_LOSS_BLOCKS, (int)grid1((long long)n * NO, LOSS_BLOCK));
+    k_loss<<<loss_blocks, LOSS_BLOCK, 0, h->stream>>>(h->y, h->t, h->d_norm, n, h->dyb, h->loss_part);
+    // dz3 = (dy W4) gelu'(z3), dz2 = (dz3 W3) gelu'(z2), dz1 = (dz2 W2) gelu'(z1)
+    // (the input gradient is not needed)
     if ((rc = gemm(h, h->dyb, NO, 1, W + OFF_W4, 1, NH, n, NH, NO, EPI_DGELU_BF16, nullptr, h->z3, nullptr, h->dz3, NH)))
         return rc;
-    // layer 3
-    if ((rc = gemm(h, h->dz3, 1, NH, h->h2, 1, NH, NH, NH, n, EPI_STORE_F32, nullptr, nullptr, G + OFF_W3, nullptr, NH)))
-        return rc;
-    k_colsum<<<1, NH, 0, h->stream>>>(h->dz3, n, NH, G + OFF_B3);
     if ((rc = gemm(h, h->dz3, NH, 1, W + OFF_W3, 1, NH, n, NH, NH, EPI_DGELU_BF16, nullptr, h->z2, nullptr, h->dz2, NH)))
         return rc;
-    // layer 2
-    if ((rc = gemm(h, h->dz2, 1, NH, h->h1, 1, NH, NH, NH, n, EPI_STORE_F32, nullptr, nullptr, G + OFF_W2, nullptr, NH)))
-        return rc;
-    k_colsum<<<1, NH, 0, h->stream>>>(h->dz2, n, NH, G + OFF_B2);
     if ((rc = gemm(h, h->dz2, NH, 1, W + OFF_W2, 1, NH, n, NH, NH, EPI_DGELU_BF16, nullptr, h->z1, nullptr, h->dz1, NH)))
         return rc;
-    // layer 1 (its input gradient is not needed)
-    if ((rc = gemm(h, h->dz1, 1, NH, h->xb, 1, NI, NH, NI, n, EPI_STORE_F32, nullptr, nullptr, G + OFF_W1, nullptr, NI)))
-        return rc;
-    k_colsum<<<1, NH, 0, h->stream>>>(h->dz1, n, NH, G + OFF_B1);
+    // every layer's dW = dz^T x and db = colsum(dz)
+    static bool configured[64] = {false};
+    const int smem = 2 * (LayerSmem<64>::A_BYTES + LayerSmem<64>::B_BYTES) + 1024;
+    if (!configured[h->device & 63]) {
+        CK(cudaFuncSetAttribute(k_weight_grads, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        configured[h->device & 63] = true;
+    }
+    WeightGradArgs a{};
+    int tiles = 0;
+    auto add = [&](int k, const __nv_bfloat16* dz, const __nv_bfloat16* x, int outs, int ins, long long ow, long long ob) {
+        a.layer[k] = WeightGrad{dz, x, outs, ins, ow, ob, tiles, (outs + GEMM_BM - 1) / GEMM_BM};
+        tiles += a.layer[k].m_tiles * ((ins + 63) / 64);
+    };
+    add(0, h->dz3, h->h2, NH, NH, OFF_W3, OFF_B3);
+    add(1, h->dz2, h->h1, NH, NH, OFF_W2, OFF_B2);
+    add(2, h->dz1, h->xb, NH, NI, OFF_W1, OFF_B1);
+    add(3, h->dyb, h->h3, NO, NH, OFF_W4, OFF_B4);
+    a.batch = n;
+    a.slice = slice_length(n);
+    a.partial = h->partial;
+    a.n_params = PARAM_STRIDE;
+    a.error = h->d_error;
+    const int slices = (n + a.slice - 1) / a.slice;
+    k_weight_grads<<<dim3(tiles, slices), GEMM_THREADS, smem, h->stream>>>(a);
+    k_reduce_params<<<grid1(NPARAM, 256), 256, 0, h->stream>>>(h->partial, slices, PARAM_STRIDE, h->loss_part, loss_blocks,
+                                                               3.0f * (float)n, h->loss, h->g, lr > 0.f, h->p, h->m, h->v,
+                                                               lr, bc1, bc2, h->wb);
     CK(cudaGetLastError());
     return DEM_MLP_OK;
 }
@@ -300,21 +329,32 @@ int dem_mlp_create(int device, int capacity, uint64_t seed, dem_mlp** out)
     if (cudaSetDevice(device) != cudaSuccess) return cleanup(DEM_MLP_ERR_CUDA);
     if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) return cleanup(DEM_MLP_ERR_CUDA);
     const size_t c = (size_t)capacity;
-    bool ok = true;
-    auto alloc = [&](auto** p, size_t count) {
-        if (ok && cudaMalloc(reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(**p)) != cudaSuccess)
-            ok = false;
+    // one device block for every array (24 allocations took most of the set-up)
+    size_t total = 0;
+    char* block = nullptr;
+    auto part = [&](auto** p, size_t count) {
+        if (block) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(block + total);
+        total += (std::max<size_t>(count, 1) * sizeof(**p) + 255) & ~(size_t)255;
     };
-    alloc(&h->d_error, 1);
-    alloc(&h->p, NPARAM); alloc(&h->g, NPARAM); alloc(&h->m, NPARAM); alloc(&h->v, NPARAM);
-    alloc(&h->wb, NPARAM);
-    alloc(&h->d_norm, 2 * NI + 2 * NO);
-    alloc(&h->x, c * NI); alloc(&h->t, c * NO); alloc(&h->xb, c * NI);
-    alloc(&h->z1, c * NH); alloc(&h->z2, c * NH); alloc(&h->z3, c * NH); alloc(&h->y, c * NO);
-    alloc(&h->h1, c * NH); alloc(&h->h2, c * NH); alloc(&h->h3, c * NH);
-    alloc(&h->dyb, c * NO); alloc(&h->dz1, c * NH); alloc(&h->dz2, c * NH); alloc(&h->dz3, c * NH);
-    alloc(&h->loss, 1);
-    if (!ok) return cleanup(fail(h, DEM_MLP_ERR_CUDA, "cudaMalloc failed"));
+    for (int pass = 0; pass < 2; ++pass) {
+        if (pass == 1) {
+            if (cudaMalloc(reinterpret_cast<void**>(&block), total) != cudaSuccess)
+                return cleanup(fail(h, DEM_MLP_ERR_CUDA, "cudaMalloc failed"));
+            h->block = block;
+            total = 0;
+        }
+        part(&h->d_error, 1);
+        part(&h->p, NPARAM); part(&h->g, NPARAM); part(&h->m, NPARAM); part(&h->v, NPARAM);
+        part(&h->wb, NPARAM);
+        part(&h->d_norm, 2 * NI + 2 * NO);
+        part(&h->x, c * NI); part(&h->t, c * NO); part(&h->xb, c * NI);
+        part(&h->z1, c * NH); part(&h->z2, c * NH); part(&h->z3, c * NH); part(&h->y, c * NO);
+        part(&h->h1, c * NH); part(&h->h2, c * NH); part(&h->h3, c * NH);
+        part(&h->dyb, c * NO); part(&h->dz1, c * NH); part(&h->dz2, c * NH); part(&h->dz3, c * NH);
+        part(&h->loss, 1);
+        part(&h->loss_part, MAX_LOSS_BLOCKS);
+        part(&h->partial, (size_t)std::min<long long>(MAX_SLICES, grid1(capacity, GEMM_BK)) * PARAM_STRIDE);
+    }
     // He-uniform weights, zero biases
     std::vector<float> p(NPARAM, 0.0f);
     std::mt19937_64 rng(seed);
@@ -386,7 +426,7 @@ int dem_mlp_forward(dem_mlp* h, const float* x, int n, float* y)
 {
     if (!h || !y) return DEM_MLP_ERR_BAD_INPUT;
     int rc;
-    if ((rc = load_batch(h, x, nullptr, n)) || (rc = forward(h, n, false))) return rc;
+    if ((rc = load_batch(h, x, nullptr, n)) || (rc = forward_fused(h, n))) return rc;
     k_denorm_outputs<<<grid1((long long)n * NO, 256), 256, 0, h->stream>>>(h->y, h->d_norm, n, h->t);
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(y, h->t, (size_t)n * NO * sizeof(float), cudaMemcpyDeviceToHost, h->stream));
@@ -407,12 +447,10 @@ int dem_mlp_train_step(dem_mlp* h, const float* x, const float* t, int n, float 
 {
     if (!h || !t || !(lr > 0.f)) return DEM_MLP_ERR_BAD_INPUT;
     int rc;
-    if ((rc = load_batch(h, x, t, n)) || (rc = forward(h, n)) || (rc = backward(h, n))) return rc;
+    const float bc1 = 1.0f - std::pow(0.9f, (float)(h->step + 1));
+    const float bc2 = 1.0f - std::pow(0.999f, (float)(h->step + 1));
+    if ((rc = load_batch(h, x, t, n)) || (rc = forward(h, n)) || (rc = backward(h, n, lr, bc1, bc2))) return rc;
     h->step += 1;
-    const float bc1 = 1.0f - std::pow(0.9f, (float)h->step);
-    const float bc2 = 1.0f - std::pow(0.999f, (float)h->step);
-    k_adam<<<grid1(NPARAM, 256), 256, 0, h->stream>>>(h->p, h->g, h->m, h->v, NPARAM, lr, bc1, bc2, h->wb);
-    CK(cudaGetLastError());
     if (loss) CK(cudaMemcpyAsync(loss, h->loss, sizeof(float), cudaMemcpyDeviceToHost, h->stream));
     return check_device_status(h);
 }
@@ -424,9 +462,9 @@ int dem_mlp_time_forward(dem_mlp* h, int n, int reps, float* ms)
     cudaEvent_t e0, e1;
     CK(cudaEventCreate(&e0));
     CK(cudaEventCreate(&e1));
-    int rc = forward(h, n, false); // warm-up
+    int rc = forward_fused(h, n); // warm-up
     CK(cudaEventRecord(e0, h->stream));
-    for (int r = 0; r < reps && !rc; ++r) rc = forward(h, n, false);
+    for (int r = 0; r < reps && !rc; ++r) rc = forward_fused(h, n);
     CK(cudaEventRecord(e1, h->stream));
     CK(cudaEventSynchronize(e1));
     float t = 0.f;
@@ -445,10 +483,7 @@ void dem_mlp_destroy(dem_mlp* h)
     if (!h) return;
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
-    void* ptrs[] = {h->d_error, h->p, h->g, h->m, h->v, h->wb, h->d_norm, h->x, h->t, h->xb, h->z1, h->z2,
-                    h->z3, h->y, h->h1, h->h2, h->h3, h->dyb, h->dz1, h->dz2, h->dz3, h->loss};
-    for (void* p : ptrs)
-        if (p) cudaFree(p);
+    if (h->block) cudaFree(h->block);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
 }

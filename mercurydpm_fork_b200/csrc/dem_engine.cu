@@ -27,7 +27,6 @@ namespace {
 constexpr unsigned FATAL_STATUS =
     (1u << DEM_ERR_CAPACITY) | (1u << DEM_ERR_NAN) | (1u << DEM_ERR_TIMEOUT) | (1u << INS_STATUS_NO_ROW);
 constexpr int GRAPH_STEPS = 16;
-constexpr int CONTROL_THREADS = 128;
 
 struct Handle {
     dem_config cfg{};
@@ -210,8 +209,9 @@ inline unsigned grid_for(long long n, int block) { return (unsigned)std::max<lon
 
 // ---- kernel launch sequences ------------------------------------------------
 // The rebuild kernel (dem_rebuild.cuh): a cooperative launch, so that its
-// grid barriers are safe; it returns at once unless the rebuild flag is set.
-cudaError_t launch_rebuild(Handle* h, cudaStream_t s)
+// grid barriers are safe; it returns at once unless the lists are out of date.
+// `step`: it opens a time step.
+cudaError_t launch_rebuild(Handle* h, cudaStream_t s, bool step)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)h->rb_grid);
@@ -223,7 +223,8 @@ cudaError_t launch_rebuild(Handle* h, cudaStream_t s)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_rebuild, h->d, h->d.rb_barrier);
+    const int move_walls = step && h->n_ins_launch == 0;
+    return cudaLaunchKernelEx(&cfg, k_rebuild, h->d, h->d.rb_barrier, step ? 1 : 0, move_walls);
 }
 constexpr int REBUILD_LAUNCHES = 1;
 
@@ -236,12 +237,14 @@ InsPtrs ins_ptrs(Handle* h)
 }
 
 // Insertion boundaries: one block per instance that has some (dem_insert.cuh),
-// after k_control and before the rebuild it may request.
+// before the rebuild it may request.
 void launch_insert(Handle* h, cudaStream_t s)
 {
-    if (h->n_ins_launch > 0)
-        k_insert<<<h->n_ins_inst, INS_THREADS, 0, s>>>(h->d, ins_ptrs(h));
+    if (h->n_ins_launch == 0) return;
+    if (h->d.n_walls > 0) k_move_walls<<<grid_for(h->d.n_walls, 128), 128, 0, s>>>(h->d);
+    k_insert<<<h->n_ins_inst, INS_THREADS, 0, s>>>(h->d, ins_ptrs(h));
 }
+int insert_launches(const Handle* h) { return h->n_ins_launch > 0 ? (h->d.n_walls > 0 ? 2 : 1) : 0; }
 constexpr int FORCE_LAUNCHES = 2;
 
 // Law variants the force kernel is instantiated for; the handle uses a
@@ -320,17 +323,16 @@ void launch_force(Handle* h, cudaStream_t s, int mode, bool last = true)
         launch_force_mode<1, false>(h, s);
 }
 
-// Captures `steps` time steps: control -> rebuild (returns at once unless
-// the skin test fired) -> force; `last`: the final step is the last of the
+// Captures `steps` time steps: rebuild (returns at once unless the skin test
+// fired) -> force; `last`: the final step is the last of the
 // dem_step call (its force evaluation writes the contact records).
 int build_graph(Handle* h, int steps, bool last, cudaGraphExec_t* out)
 {
     cudaStream_t s = h->stream;
     CU(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < steps; ++k) {
-        k_control<<<1, CONTROL_THREADS, 0, s>>>(h->d_ctl, h->d.walls, h->d_wgeom, h->d.n_walls, h->d.dt);
         launch_insert(h, s);
-        const cudaError_t e = launch_rebuild(h, s);
+        const cudaError_t e = launch_rebuild(h, s, true);
         if (e != cudaSuccess) {
             cudaGraph_t g = nullptr;
             cudaStreamEndCapture(s, &g);
@@ -1392,10 +1394,7 @@ static int ensure_lists(Handle* h)
     int rc = read_control(h, &c);
     if (rc) return rc;
     if (!c.force_rebuild) return DEM_OK;
-    c.rebuild = 1;
-    c.force_rebuild = 0;
-    CU(cudaMemcpyAsync(h->d_ctl, &c, sizeof(Control), cudaMemcpyHostToDevice, h->stream));
-    CU(launch_rebuild(h, h->stream));
+    CU(launch_rebuild(h, h->stream, false));
     return read_control(h, &c);
 }
 
@@ -1522,21 +1521,18 @@ int dem_step(dem_handle* hh, int nsteps)
     if (h->initial_pending && d.n > 0) {
         // DPMBase::initialiseSolve: first force evaluation at the uploaded state.
         // If dem_upload_contacts already built the lists, they are kept.
-        c0.rebuild = c0.force_rebuild ? 1 : 0;
-        c0.force_rebuild = 0;
-        c0.pending_flip = 1;
+        c0.view = StepView{c0.cur, c0.lbuf, c0.hcur, c0.pcur, 1, 0};
     }
     CU(cudaMemcpyAsync(h->d_ctl, &c0, sizeof(Control), cudaMemcpyHostToDevice, h->stream));
     CU(cudaEventRecord(h->ev0, h->stream));
     if (d.n > 0) {
         if (h->initial_pending) {
-            if (c0.rebuild) {
-                CU(launch_rebuild(h, h->stream));
+            if (c0.force_rebuild) {
+                CU(launch_rebuild(h, h->stream, false));
                 launches += REBUILD_LAUNCHES;
             }
             launch_force(h, h->stream, 0);
-            k_flip<<<1, 32, 0, h->stream>>>(h->d_ctl);
-            launches += force_launches(h) + 1;
+            launches += force_launches(h);
             CU(cudaGetLastError());
             h->initial_pending = false;
         }
@@ -1558,19 +1554,16 @@ int dem_step(dem_handle* hh, int nsteps)
                 }
                 while (left-- > 0) CU(cudaGraphLaunch(h->graph1, h->stream));
                 CU(cudaGraphLaunch(h->graphF, h->stream));
-                launches += (1ll + REBUILD_LAUNCHES + force_launches(h) + (h->n_ins_launch > 0)) * nsteps;
+                launches += (REBUILD_LAUNCHES + force_launches(h) + insert_launches(h)) * (long long)nsteps;
             } else {
                 for (int k = 0; k < nsteps; ++k) {
-                    k_control<<<1, CONTROL_THREADS, 0, h->stream>>>(h->d_ctl, d.walls, h->d_wgeom, d.n_walls, d.dt);
                     launch_insert(h, h->stream);
-                    CU(launch_rebuild(h, h->stream));
+                    CU(launch_rebuild(h, h->stream, true));
                     launch_force(h, h->stream, 1, k == nsteps - 1);
                 }
                 CU(cudaGetLastError());
-                launches += (1ll + force_launches(h) + REBUILD_LAUNCHES + (h->n_ins_launch > 0)) * nsteps;
+                launches += (REBUILD_LAUNCHES + force_launches(h) + insert_launches(h)) * (long long)nsteps;
             }
-            k_flip<<<1, 32, 0, h->stream>>>(h->d_ctl);
-            launches += 1;
         }
     }
     CU(cudaEventRecord(h->ev1, h->stream));
@@ -2008,9 +2001,8 @@ int dem_time_force_kernel(dem_handle* hh, int reps, double* ms_per_launch)
     // the spare buffers; nothing is flipped, so the state stays as it was
     Control probe = saved;
     probe.spare = 1;
-    probe.final_step = 0;
-    probe.first_step = 0;
-    probe.pending_flip = 0;
+    // as the next step would read the buffers
+    probe.view = StepView{saved.cur, saved.lbuf, saved.hcur ^ saved.pending_flip, saved.pcur ^ saved.pending_flip, 0, 0};
     probe.record = 0;
     CU(cudaMemcpyAsync(h->d_ctl, &probe, sizeof(Control), cudaMemcpyHostToDevice, h->stream));
     launch_force(h, h->stream, 1, false); // warm-up
@@ -2087,9 +2079,8 @@ int dem_autotune(dem_handle* hh, int reps, dem_tuning* out)
     if (rc) return rc;
     Control probe = saved;
     probe.spare = 1;
-    probe.final_step = 0;
-    probe.first_step = 0;
-    probe.pending_flip = 0;
+    // as the next step would read the buffers
+    probe.view = StepView{saved.cur, saved.lbuf, saved.hcur ^ saved.pending_flip, saved.pcur ^ saved.pending_flip, 0, 0};
     probe.record = 0;
     CU(cudaMemcpyAsync(h->d_ctl, &probe, sizeof(Control), cudaMemcpyHostToDevice, h->stream));
     const dem_tuning start = h->tune;

@@ -119,19 +119,27 @@ struct ContactRecord {
     double springs[9];
 };
 
+// What the kernels of one force evaluation read: written by one thread of
+// k_rebuild (or the host) before it, when all of that launch's blocks decide
+// from the fields below, which k_units then advances.
+struct StepView {
+    int cur, lbuf, hcur, pcur; // state, unit-list, uidx and pool buffers to read
+    int final_step;            // this step is the last of the dem_step call
+    int first_step;            // this step is the first after the initial evaluation
+};
+
 struct Control {
+    StepView view;
+    double next_disp_acc;  // disp_acc once this step is under way
     int cur;               // state buffer holding the current state
     int lbuf;              // unit-list buffer in use
     int pending_flip;      // the last force evaluation wrote the other spring pool and uidx
-    int rebuild;           // this step rebuilds the neighbour list
-    int final_step;        // this step is the last of the dem_step call
-    int force_rebuild;     // rebuild at the next control point regardless of displacement
+    int force_rebuild;     // rebuild before the next evaluation regardless of displacement
     int record;            // record contacts at final/initial evaluations
     int spare;             // 1: k_sum writes the other state buffer (timing launches; the state stays)
     long long steps_left;
     long long n_rebuilds;
     long long steps_done;  // time steps since the upload
-    int first_step;        // this step is the first after the initial evaluation
     int hcur;              // uidx (and triangle history) buffer of the last evaluation
     double disp_acc;       // sum of per-step maximum displacements since the last rebuild
     double skin;
@@ -194,8 +202,8 @@ struct DevPtrs {
     // tables
     const InstanceDev *inst;
     const dem_species_pair *species;
-    dem_wall *walls;         // moved by k_control every step
-    const WallGeom *wgeom;   // per wall; faces, edges and corners of intersection walls
+    dem_wall *walls;         // moved before every step's force evaluation (move_wall)
+    WallGeom *wgeom;   // per wall; faces, edges and corners of intersection walls
     int n_walls;
     int n_instances;
     // triangle-wall items of one evaluation: (particle, item, wall bits, 0)

@@ -11,7 +11,7 @@
 // reference's order, and the whole block tests each candidate (walls, the
 // particles of the cells around the candidate and its periodic images, the
 // particles placed earlier in the same launch). It runs in every time step
-// after k_control (walls moved, state buffers flipped) and before the
+// after the drift (k_move_walls) and before the
 // rebuild, which it requests when it placed a particle: that is the
 // reference's place in DPMBase::computeOneTimeStep (after the drift, before
 // the forces, DPMBase.cc:4348-4352).
@@ -260,7 +260,7 @@ __global__ void __launch_bounds__(INS_THREADS) k_insert(DevPtrs d, InsPtrs ip)
     const double next_time = S.time + d.dt; // DPMBase::getNextTime
     // reach of the cell search beyond r_c + r_t + interaction distance: the
     // largest displacement since the rebuild (with room for its rounding)
-    const double disp = ctl->disp_acc * (1.0 + 1e-9);
+    const double disp = spent_skin(ctl) * (1.0 + 1e-9);
     double rmax = 0.0;
     for (int l = 0; l < I.n_levels; ++l) rmax = fmax(rmax, I.level_rmax[l]);
     __syncthreads();
@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(INS_THREADS) k_insert(DevPtrs d, InsPtrs ip)
         S.filed_from = first_row;
         S.next_row = s_next_row;
         S.time = next_time; // DPMBase::time_ += timeStep_ at the end of the step
-        if (s_placed) ctl->rebuild = 1; // the new particles need cells and lists
+        if (s_placed) ctl->force_rebuild = 1; // the new particles need cells and lists
     }
 }
 

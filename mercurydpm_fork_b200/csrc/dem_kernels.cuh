@@ -1,13 +1,11 @@
 // dem_kernels.cuh -- the DEM time-step kernels.
 //
 // Per time step (captured in a CUDA graph):
-//   k_control   moves the walls (one thread per wall); one thread applies
-//               the pending state-buffer flip, adds the last step's maximum
-//               displacement to the skin budget and sets the rebuild flag
+//   k_rebuild   one cooperative kernel, launched every step: moves the walls
+//               and returns at once unless the skin budget is spent
 //               (MercuryBase::hGridNeedsRebuilding, MercuryBase.cc:496-535,
-//               turned into a Verlet-skin test).
-//   k_rebuild   one cooperative kernel, launched every step and returning at
-//               once unless the flag is set (dem_rebuild.cuh): cell keys per
+//               turned into a Verlet-skin test), which every block decides for
+//               itself (dem_rebuild.cuh). A rebuild: cell keys per
 //               HGrid level, counting sort, per-cell ordering by particle id,
 //               permutation gather of the state, neighbour lists with
 //               contact-history carry-over, their reverse index (replaces
@@ -31,53 +29,35 @@ __device__ __forceinline__ V3 xyz(double4 a) { return V3{a.x, a.y, a.z}; }
 // ---------------------------------------------------------------------------
 // control
 // ---------------------------------------------------------------------------
-__global__ void k_control(Control* ctl, dem_wall* walls, WallGeom* wgeom, int n_walls, double dt)
+// Walls move before the force evaluation of every step, after the particles
+// (DPMBase::integrateBeforeForceComputation, DPMBase.cc:3228-3261, through
+// BaseInteractable::integrateBeforeForceComputation, BaseInteractable.cc:538-600:
+// move(v dt), then rotate(omega dt) = Quaternion::updateAngularDisplacement).
+// A triangle wall then recomputes its vertices and normals
+// (TriangleWall::move / rotate -> updateVertexAndNormal).
+__device__ __forceinline__ void move_wall(dem_wall& w, WallGeom& geom, double dt)
 {
-    // Walls move before the force evaluation of every step, after the particles
-    // (DPMBase::integrateBeforeForceComputation, DPMBase.cc:3228-3261, through
-    // BaseInteractable::integrateBeforeForceComputation, BaseInteractable.cc:538-600:
-    // move(v dt), then rotate(omega dt) = Quaternion::updateAngularDisplacement).
-    // A triangle wall then recomputes its vertices and normals
-    // (TriangleWall::move / rotate -> updateVertexAndNormal).
-    for (int k = threadIdx.x; k < n_walls; k += blockDim.x) {
-        dem_wall& w = walls[k];
-        for (int a = 0; a < 3; ++a) w.position[a] += w.velocity[a] * dt;
-        const Q4 q = quat_rotate(Q4{w.orientation[0], w.orientation[1], w.orientation[2], w.orientation[3]},
-                                 v3(w.angular_velocity[0] * dt, w.angular_velocity[1] * dt, w.angular_velocity[2] * dt));
-        w.orientation[0] = q.q0; w.orientation[1] = q.q1; w.orientation[2] = q.q2; w.orientation[3] = q.q3;
-        const bool still = w.velocity[0] == 0.0 && w.velocity[1] == 0.0 && w.velocity[2] == 0.0 &&
-                           w.angular_velocity[0] == 0.0 && w.angular_velocity[1] == 0.0 &&
-                           w.angular_velocity[2] == 0.0; // nothing moved: the geometry stands
-        if (w.type == DEM_WALL_TRIANGLE && !still) triangle_geometry(w, wgeom[k]);
-    }
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (ctl->pending_flip) { // a force evaluation wrote the other spring pool and uidx
-        ctl->hcur ^= 1;
-        ctl->pcur ^= 1;
-        ctl->pending_flip = 0;
-    }
-    const double d = sqrt(__longlong_as_double((long long)ctl->step_disp2_bits));
-    ctl->step_disp2_bits = 0ull;
-    ctl->disp_acc += d;
-    const int rebuild = ctl->force_rebuild || (2.0 * ctl->disp_acc >= ctl->skin);
-    ctl->rebuild = rebuild;
-    ctl->force_rebuild = 0;
-    ctl->final_step = (ctl->steps_left <= 1);
-    ctl->steps_left -= 1;
-    if (ctl->final_step) ctl->n_records = 0; // records describe the last evaluation only
-    ctl->first_step = (ctl->steps_done == 0);
-    ctl->steps_done += 1;
-    ctl->pending_flip = 1; // the force evaluation of this step writes the other pool
+    for (int a = 0; a < 3; ++a) w.position[a] += w.velocity[a] * dt;
+    const Q4 q = quat_rotate(Q4{w.orientation[0], w.orientation[1], w.orientation[2], w.orientation[3]},
+                             v3(w.angular_velocity[0] * dt, w.angular_velocity[1] * dt, w.angular_velocity[2] * dt));
+    w.orientation[0] = q.q0; w.orientation[1] = q.q1; w.orientation[2] = q.q2; w.orientation[3] = q.q3;
+    const bool still = w.velocity[0] == 0.0 && w.velocity[1] == 0.0 && w.velocity[2] == 0.0 &&
+                       w.angular_velocity[0] == 0.0 && w.angular_velocity[1] == 0.0 &&
+                       w.angular_velocity[2] == 0.0; // nothing moved: the geometry stands
+    if (w.type == DEM_WALL_TRIANGLE && !still) triangle_geometry(w, geom);
 }
 
-__global__ void k_flip(Control* ctl)
+// With insertion boundaries the walls move before them, in a launch of their own.
+__global__ void __launch_bounds__(128) k_move_walls(DevPtrs d)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    if (ctl->pending_flip) { // a force evaluation wrote the other spring pool and uidx
-        ctl->hcur ^= 1;
-        ctl->pcur ^= 1;
-        ctl->pending_flip = 0;
-    }
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w < d.n_walls) move_wall(d.walls[w], d.wgeom[w], d.dt);
+}
+
+// The skin budget spent since the last rebuild, the last drift included.
+__device__ __forceinline__ double spent_skin(const Control* ctl)
+{
+    return ctl->disp_acc + sqrt(__longlong_as_double((long long)ctl->step_disp2_bits));
 }
 
 // ---------------------------------------------------------------------------

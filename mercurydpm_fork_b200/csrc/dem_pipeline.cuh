@@ -350,10 +350,22 @@ __global__ void __launch_bounds__(UNIT_BLOCK, MINB) k_units(const __grid_constan
     __shared__ unsigned short hit_of[UNIT_CHUNK_MAX];
     __shared__ int n_hit, item0;
     Control* ctl = d.ctl;
-    const int c = ctl->cur, l = ctl->lbuf, hc = ctl->hcur, hn = hc ^ 1, pc = ctl->pcur;
-    const bool final_step = (MODE == 0) ? true : (ctl->final_step != 0);
-    const bool record = RECORD && final_step && ctl->record;
-    const bool first = (MODE == 1) && ctl->first_step;
+    const StepView& view = ctl->view;
+    const int c = view.cur, l = view.lbuf, hc = view.hcur, hn = hc ^ 1, pc = view.pcur;
+    const bool record = RECORD && (MODE == 0 || view.final_step) && ctl->record;
+    const bool first = (MODE == 1) && view.first_step;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && !ctl->spare) { // no kernel of this evaluation reads these
+        ctl->hcur = hc;
+        ctl->pcur = pc;
+        ctl->pending_flip = 1; // this evaluation writes the other pool and uidx
+        ctl->force_rebuild = 0;
+        if (MODE == 1) {
+            ctl->disp_acc = ctl->next_disp_acc;
+            ctl->step_disp2_bits = 0ull;
+            ctl->steps_left -= 1;
+            ctl->steps_done += 1;
+        }
+    }
     const int n_units = min(ctl->n_units, d.unit_cap);
     const double dt = d.dt;
     stage_tables(d, tables);
@@ -615,10 +627,9 @@ __global__ void __launch_bounds__(TRI_BLOCK) k_tri(DevPtrs d)
     constexpr int MAXT = DEM_MAX_TRIANGLE_CONTACTS;
     static_assert(NCOMP % 2 == 1, "the pad word of a history row holds the creation key");
     Control* ctl = d.ctl;
-    const int c = ctl->cur, hc = ctl->hcur, hn = hc ^ 1;
-    const bool final_step = (MODE == 0) ? true : (ctl->final_step != 0);
-    const bool record = final_step && ctl->record;
-    const bool first = (MODE == 1) && ctl->first_step;
+    const int c = ctl->view.cur, hc = ctl->view.hcur, hn = hc ^ 1;
+    const bool record = (MODE == 0 || ctl->view.final_step) && ctl->record;
+    const bool first = (MODE == 1) && ctl->view.first_step;
     const int n_tri = min((int)ctl->n_tri, d.n);
     const double dt = d.dt;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_tri; t += gridDim.x * blockDim.x) {
@@ -808,9 +819,9 @@ __global__ void __launch_bounds__(BLOCK, SUM_THREADS_PER_SM / BLOCK) k_sum(DevPt
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     Control* ctl = d.ctl;
-    const int c = ctl->cur, to = c ^ ctl->spare;
-    const int* uidx = d.uidx[ctl->hcur ^ 1]; // of this evaluation
-    const bool final_step = (MODE == 0) ? true : (ctl->final_step != 0);
+    const int c = ctl->view.cur, to = c ^ ctl->spare;
+    const int* uidx = d.uidx[ctl->view.hcur ^ 1]; // of this evaluation
+    const bool final_step = (MODE == 0) ? true : (ctl->view.final_step != 0);
     const double dt = d.dt;
     if (s == 0) { // k_units and k_tri are done: the next evaluation starts new lists
         // the springs kept at the pool top in the first time step must not have

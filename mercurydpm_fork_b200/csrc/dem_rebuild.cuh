@@ -1,12 +1,17 @@
 // dem_rebuild.cuh -- the neighbour-list rebuild as one cooperative kernel.
 //
-// k_rebuild is launched after k_control in every time step (a cooperative
-// launch: all its blocks are resident together) and returns at once unless
-// k_control set the rebuild flag (the Verlet-skin test restating
-// MercuryBase::hGridNeedsRebuilding, MercuryBase.cc:496-535). One launch that
-// usually does nothing costs less than a graph conditional node around ten
-// kernels. When the flag is set, the blocks run the steps below in turn,
-// separated by grid barriers:
+// k_rebuild opens every time step (a cooperative launch: all its blocks are
+// resident together). It moves the walls, and every block decides from the same
+// fields of the control record, which no thread of this launch writes unless it
+// rebuilds, whether the skin budget is spent (the Verlet-skin test restating
+// MercuryBase::hGridNeedsRebuilding, MercuryBase.cc:496-535); if not, it returns
+// at once. One thread writes the step's view of the buffers (StepView). A
+// control kernel of its own before it cost 2 to 3 us of a step, and 21 us with
+// the 1,024 walls of a batch on its one block; deciding in k_sum's last block
+// instead held every block of it at a fence (a step of the 1,000,000 drum 6 %
+// slower). One launch that usually does nothing costs less than a graph
+// conditional node around ten kernels. When the budget is spent, the blocks run
+// the steps below in turn, separated by grid barriers:
 //
 //   1 cell keys per HGrid level and counts per cell         (keys_one)
 //   2 exclusive scan of the counts, one chunk of cells per block
@@ -115,14 +120,36 @@ __device__ __forceinline__ int block_sum(int v, int* warp_sums)
     return total;
 }
 
-__global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned long long* barrier_ctr)
+// step: 1 the launch opens a time step; 0 it only brings the lists up to date
+// (before the initial evaluation). move_walls: they have not moved yet.
+__global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned long long* barrier_ctr, int step,
+                                                         int move_walls)
 {
     Control* ctl = d.ctl;
-    if (!ctl->rebuild) return;
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
+    // read by every block before the first barrier
+    const int flip = ctl->pending_flip;
+    const int hc = ctl->cur, lo = ctl->lbuf, hh = ctl->hcur ^ flip;
+    const double spent = step ? spent_skin(ctl) : 0.0;
+    const bool go = ctl->force_rebuild || (step && 2.0 * spent >= ctl->skin);
+    if (move_walls)
+        for (int w = gt; w < d.n_walls; w += gs) move_wall(d.walls[w], d.wgeom[w], d.dt);
+    if (gt == 0) {
+        StepView& v = ctl->view;
+        v.pcur = ctl->pcur ^ flip;
+        v.final_step = !step || ctl->steps_left <= 1;
+        v.first_step = step && ctl->steps_done == 0;
+        if (step && v.final_step) ctl->n_records = 0; // records describe the last evaluation only
+        if (!go) {
+            v.cur = hc;
+            v.lbuf = lo;
+            v.hcur = hh;
+            ctl->next_disp_acc = spent;
+        }
+    }
+    if (!go) return;
     __shared__ unsigned long long base_s;
     __shared__ int warp_sums[RB_BLOCK / 32];
-    // read by every block before the first barrier
-    const int hc = ctl->cur, lo = ctl->lbuf, hh = ctl->hcur;
     const int old_units = min(ctl->n_units, d.unit_cap);
     if (threadIdx.x == 0) {
         const unsigned long long per = (unsigned long long)gridDim.x * RB_BARRIERS;
@@ -130,7 +157,6 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
     }
     __syncthreads();
     GridBarrier g{barrier_ctr, base_s, 0u};
-    const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
 
     if (blockIdx.x == 0 && threadIdx.x == 0) ctl->n_units_next = 0;
 
@@ -202,11 +228,15 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
             if (!d.wact[hh ^ 1][s]) d.wact[hh][s] = 0u;
 
     if (blockIdx.x == 0 && threadIdx.x == 0) { // the gathered state and the new lists become current
-        ctl->cur = hc ^ 1;
-        ctl->lbuf = lo ^ 1;
-        ctl->hcur = hh ^ 1;
+        StepView& v = ctl->view;
+        v.cur = ctl->cur = hc ^ 1;
+        v.lbuf = ctl->lbuf = lo ^ 1;
+        v.hcur = ctl->hcur = hh ^ 1;
+        ctl->pcur = v.pcur;
+        ctl->pending_flip = 0;
         ctl->n_units = min(ctl->n_units_next, d.unit_cap);
-        ctl->disp_acc = 0.0;
+        ctl->disp_acc = ctl->next_disp_acc = 0.0;
+        ctl->force_rebuild = 0;
         ctl->n_rebuilds += 1;
     }
 }

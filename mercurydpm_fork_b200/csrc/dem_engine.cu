@@ -1149,7 +1149,7 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
         d.cnt = kept.cnt; d.own = kept.own; d.wcand = kept.wcand; d.ubase = kept.ubase; d.wbase = kept.wbase;
         d.epair = kept.epair;
         d.force = kept.force; d.torque = kept.torque; d.key = kept.key; d.perm = kept.perm; d.newidx = kept.newidx;
-        d.cell_count = kept.cell_count; d.cell_start = kept.cell_start; d.cell_cursor = kept.cell_cursor;
+        d.cell_count = kept.cell_count; d.cell_start = kept.cell_start;
         d.block_sums = kept.block_sums; d.rb_barrier = kept.rb_barrier; d.inst = kept.inst; d.species = kept.species; d.walls = kept.walls;
         d.wgeom = kept.wgeom; d.n_walls = kept.n_walls; d.ctl = kept.ctl; d.records = kept.records;
         d.n_instances = kept.n_instances;
@@ -1205,7 +1205,6 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
     if ((rc = dalloc(h, &d.newidx, NC))) return rc;
     if ((rc = dalloc(h, &d.cell_count, (size_t)ncells + 1))) return rc;
     if ((rc = dalloc(h, &d.cell_start, (size_t)ncells + 1))) return rc;
-    if ((rc = dalloc(h, &d.cell_cursor, (size_t)ncells + 1))) return rc;
     if ((rc = dalloc(h, &d.block_sums, (size_t)h->rb_grid + 1))) return rc;
     if ((rc = dalloc(h, &d.rb_barrier, 1))) return rc;
     if ((rc = dalloc(h, &h->d_inst, h->inst.size()))) return rc;

@@ -195,7 +195,7 @@ struct DevPtrs {
     double *whist[2];        // triangle walls: springs and creation key per (particle, wall)
     unsigned int *wact[2];   // triangle walls: which of them hold a contact's history
     // broad phase scratch
-    int *key, *perm, *newidx, *cell_count, *cell_start, *cell_cursor, *block_sums;
+    int *key, *perm, *newidx, *cell_count, *cell_start, *block_sums;
     unsigned long long *rb_barrier; // arrivals at the rebuild's grid barriers (only grows)
     float4 *pf;              // (x, y, z, r) in FP32 of the gathered state: the list build's prefilter
     int *row_slot;           // caller row -> slot of the current order (insertion boundaries only, else null)

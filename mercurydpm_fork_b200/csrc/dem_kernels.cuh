@@ -103,22 +103,27 @@ __device__ __forceinline__ void keys_one(const DevPtrs& d, int i, int c)
     atomicAdd(&d.cell_count[key], 1);
 }
 
-// Slot of particle i in the counting sort.
+// Slot of particle i in the counting sort. The counts go back to zero for the
+// next rebuild. The particle that takes its cell's first slot orders the cell
+// (cell_sort_one): its key turns negative.
 __device__ __forceinline__ void scatter_one(const DevPtrs& d, int i)
 {
     const int key = d.key[i];
-    const int slot = d.cell_start[key] + atomicAdd(&d.cell_cursor[key], 1);
-    d.perm[slot] = i;
+    const int left = atomicSub(&d.cell_count[key], 1) - 1;
+    d.perm[d.cell_start[key] + left] = i;
+    if (left == 0) d.key[i] = ~key;
 }
 
-// Orders the members of every cell by particle id, so the sorted order (and
-// with it every neighbour list and force sum) does not depend on the order in
-// which the atomics above were served. Resets the counters for the next rebuild.
-__device__ __forceinline__ void cell_sort_one(const DevPtrs& d, int cell, int c)
+// Orders the members of a cell by particle id, so the sorted order (and with it
+// every neighbour list and force sum) does not depend on the order in which the
+// atomics above were served. By particle, not by cell: most cells of a sparse
+// grid are empty.
+__device__ __forceinline__ void cell_sort_one(const DevPtrs& d, int i, int c)
 {
-    const int b = d.cell_start[cell], e = d.cell_start[cell + 1];
-    d.cell_count[cell] = 0;
-    d.cell_cursor[cell] = 0;
+    const int cell = ~d.key[i];
+    if (cell < 0) return; // another particle of the cell has it
+    const int b = d.cell_start[cell];
+    const int e = d.cell_start[cell + 1];
     if (e - b < 2 || cell == d.ncells - 1) return; // the graveyard is not ordered
     if (e - b > 512) { // pathological pile-up (e.g. particles far outside the grid)
         atomicOr(&d.ctl->status, 1u << DEM_ERR_DOMAIN);

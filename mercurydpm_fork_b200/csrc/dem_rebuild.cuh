@@ -14,8 +14,8 @@
 // the steps below in turn, separated by grid barriers:
 //
 //   1 cell keys per HGrid level and counts per cell         (keys_one)
-//   2 exclusive scan of the counts, one chunk of cells per block
-//   3 chunk offsets (each block sums the totals before it)
+//   2 total of the counts of one chunk of cells per block
+//   3 exclusive scan of the chunk from the sum of the totals before it
 //   4 counting-sort scatter                                 (scatter_one)
 //   5 per-cell ordering by particle id, counters reset      (cell_sort_one)
 //   6 permutation gather of the state                       (gather_one)
@@ -164,28 +164,69 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
     for (int i = gt; i < d.n; i += gs) keys_one(d, i, hc);
     if (!grid_barrier(g, ctl)) return;
 
-    // 2 exclusive scan of this block's chunk of cells
-    const int chunk = (d.ncells + gridDim.x - 1) / gridDim.x;
-    const int c0 = min(d.ncells, blockIdx.x * chunk), c1 = min(d.ncells, c0 + chunk);
-    int carry = 0;
-    for (int t0 = c0; t0 < c1; t0 += RB_BLOCK) {
-        const int i = t0 + threadIdx.x;
-        const int v = i < c1 ? d.cell_count[i] : 0;
-        int tile_total;
-        const int ex = block_exclusive_scan(v, warp_sums, tile_total);
-        if (i < c1) d.cell_start[i] = carry + ex;
-        carry += tile_total;
-        __syncthreads(); // warp_sums is reused by the next tile
+    // 2 total of this block's chunk of cells. A thread takes 16 cells of a tile in
+    // 16-byte loads: a batch of 1,024 heaps has 22 million cells, mostly empty, and
+    // a tile of one cell a thread made 195 dependent steps of 2 and 3.
+    constexpr int PER = 16, TILE = PER * RB_BLOCK;
+    const int tiles = (d.ncells + TILE - 1) / TILE;
+    const int per_block = (tiles + gridDim.x - 1) / gridDim.x;
+    const long long c0 = min((long long)d.ncells, (long long)blockIdx.x * per_block * TILE);
+    const long long c1 = min((long long)d.ncells, c0 + (long long)per_block * TILE);
+    auto load16 = [&](long long at, int (&v)[PER]) {
+        if (at + PER <= c1) {
+            const int4* p = reinterpret_cast<const int4*>(d.cell_count + at); // at: a multiple of 16
+#pragma unroll
+            for (int q = 0; q < PER / 4; ++q) {
+                const int4 x = p[q];
+                v[4 * q] = x.x; v[4 * q + 1] = x.y; v[4 * q + 2] = x.z; v[4 * q + 3] = x.w;
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < PER; ++q) v[q] = at + q < c1 ? d.cell_count[at + q] : 0;
+        }
+    };
+    int total = 0;
+    for (long long t0 = c0; t0 < c1; t0 += TILE) {
+        int v[PER];
+        load16(t0 + (long long)threadIdx.x * PER, v);
+#pragma unroll
+        for (int q = 0; q < PER; ++q) total += v[q];
     }
-    if (threadIdx.x == 0) d.block_sums[blockIdx.x] = carry;
+    total = block_sum(total, warp_sums);
+    if (threadIdx.x == 0) d.block_sums[blockIdx.x] = total;
     if (!grid_barrier(g, ctl)) return;
 
-    // 3 offsets of the chunks
+    // 3 scan from the totals of the chunks before
     int part = 0;
     for (int b = threadIdx.x; b < (int)blockIdx.x; b += RB_BLOCK) part += d.block_sums[b];
-    const int off = block_sum(part, warp_sums);
-    for (int i = c0 + threadIdx.x; i < c1; i += RB_BLOCK) d.cell_start[i] += off;
-    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) d.cell_start[d.ncells] = off + carry;
+    int before = block_sum(part, warp_sums);
+    for (long long t0 = c0; t0 < c1; t0 += TILE) {
+        const long long at = t0 + (long long)threadIdx.x * PER;
+        int v[PER], mine = 0;
+        load16(at, v);
+#pragma unroll
+        for (int q = 0; q < PER; ++q) mine += v[q];
+        int tile_total;
+        int run = before + block_exclusive_scan(mine, warp_sums, tile_total);
+#pragma unroll
+        for (int q = 0; q < PER; ++q) {
+            const int x = v[q];
+            v[q] = run;
+            run += x;
+        }
+        if (at + PER <= c1) {
+            int4* p = reinterpret_cast<int4*>(d.cell_start + at);
+#pragma unroll
+            for (int q = 0; q < PER / 4; ++q) p[q] = make_int4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        } else {
+#pragma unroll
+            for (int q = 0; q < PER; ++q)
+                if (at + q < c1) d.cell_start[at + q] = v[q];
+        }
+        before += tile_total;
+        __syncthreads(); // warp_sums is reused by the next tile
+    }
+    if (c0 < c1 && c1 == d.ncells && threadIdx.x == 0) d.cell_start[d.ncells] = before;
     if (!grid_barrier(g, ctl)) return;
 
     // 4 scatter
@@ -193,7 +234,7 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
     if (!grid_barrier(g, ctl)) return;
 
     // 5 id order inside each cell
-    for (int cell = gt; cell < d.ncells; cell += gs) cell_sort_one(d, cell, hc);
+    for (int i = gt; i < d.n; i += gs) cell_sort_one(d, i, hc);
     if (!grid_barrier(g, ctl)) return;
 
     // 6 gather

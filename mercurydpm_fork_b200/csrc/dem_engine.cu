@@ -223,8 +223,7 @@ cudaError_t launch_rebuild(Handle* h, cudaStream_t s, bool step)
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const int move_walls = step && h->n_ins_launch == 0;
-    return cudaLaunchKernelEx(&cfg, k_rebuild, h->d, h->d.rb_barrier, step ? 1 : 0, move_walls);
+    return cudaLaunchKernelEx(&cfg, k_rebuild, h->d, h->d.rb_barrier, step ? 1 : 0);
 }
 constexpr int REBUILD_LAUNCHES = 1;
 
@@ -240,11 +239,15 @@ InsPtrs ins_ptrs(Handle* h)
 // before the rebuild it may request.
 void launch_insert(Handle* h, cudaStream_t s)
 {
-    if (h->n_ins_launch == 0) return;
-    if (h->d.n_walls > 0) k_move_walls<<<grid_for(h->d.n_walls, 128), 128, 0, s>>>(h->d);
-    k_insert<<<h->n_ins_inst, INS_THREADS, 0, s>>>(h->d, ins_ptrs(h));
+    if (h->n_ins_launch > 0)
+        k_insert<<<h->n_ins_inst, INS_THREADS, 0, s>>>(h->d, ins_ptrs(h));
 }
-int insert_launches(const Handle* h) { return h->n_ins_launch > 0 ? (h->d.n_walls > 0 ? 2 : 1) : 0; }
+int insert_launches(const Handle* h) { return h->n_ins_launch > 0 ? 1 : 0; }
+// blocks over the particles, and after them over the walls
+unsigned grid_with_walls(const Handle* h, int block)
+{
+    return grid_for(h->d.n, block) + (unsigned)((h->d.n_walls + block - 1) / block);
+}
 constexpr int FORCE_LAUNCHES = 2;
 
 // Law variants the force kernel is instantiated for; the handle uses a
@@ -278,9 +281,9 @@ void launch_pipeline(Handle* h, cudaStream_t s)
     }
     if (h->kev) cudaEventRecord(h->kev[1], s);
     switch (h->tune.sum_block) {
-    case 64: k_sum<MODE, 64><<<grid_for(d.n, 64), 64, 0, s>>>(d); break;
-    case 256: k_sum<MODE, 256><<<grid_for(d.n, 256), 256, 0, s>>>(d); break;
-    default: k_sum<MODE, SUM_BLOCK><<<grid_for(d.n, SUM_BLOCK), SUM_BLOCK, 0, s>>>(d);
+    case 64: k_sum<MODE, 64><<<grid_with_walls(h, 64), 64, 0, s>>>(d); break;
+    case 256: k_sum<MODE, 256><<<grid_with_walls(h, 256), 256, 0, s>>>(d); break;
+    default: k_sum<MODE, SUM_BLOCK><<<grid_with_walls(h, SUM_BLOCK), SUM_BLOCK, 0, s>>>(d);
     }
     if (h->kev) cudaEventRecord(h->kev[2], s);
 }
@@ -1538,7 +1541,7 @@ int dem_step(dem_handle* hh, int nsteps)
         if (nsteps > 0) {
             long long sl = nsteps;
             CU(cudaMemcpyAsync(&h->d_ctl->steps_left, &sl, sizeof(long long), cudaMemcpyHostToDevice, h->stream));
-            k_kick_drift<<<grid_for(d.n, 256), 256, 0, h->stream>>>(d);
+            k_kick_drift<<<grid_with_walls(h, 256), 256, 0, h->stream>>>(d);
             launches += 1;
             if (h->cfg.use_graphs) {
                 if (!h->graph1) {

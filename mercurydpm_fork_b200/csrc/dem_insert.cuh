@@ -11,7 +11,7 @@
 // reference's order, and the whole block tests each candidate (walls, the
 // particles of the cells around the candidate and its periodic images, the
 // particles placed earlier in the same launch). It runs in every time step
-// after the drift (k_move_walls) and before the
+// after the drift (and the walls) and before the
 // rebuild, which it requests when it placed a particle: that is the
 // reference's place in DPMBase::computeOneTimeStep (after the drift, before
 // the forces, DPMBase.cc:4348-4352).

@@ -1,9 +1,8 @@
 // dem_kernels.cuh -- the DEM time-step kernels.
 //
 // Per time step (captured in a CUDA graph):
-//   k_rebuild   one cooperative kernel, launched every step: moves the walls
-//               and returns at once unless the skin budget is spent
-//               (MercuryBase::hGridNeedsRebuilding, MercuryBase.cc:496-535,
+//   k_rebuild   one cooperative kernel, launched every step: returns at once
+//               unless the skin budget is spent (MercuryBase::hGridNeedsRebuilding, MercuryBase.cc:496-535,
 //               turned into a Verlet-skin test), which every block decides for
 //               itself (dem_rebuild.cuh). A rebuild: cell keys per
 //               HGrid level, counting sort, per-cell ordering by particle id,
@@ -47,11 +46,13 @@ __device__ __forceinline__ void move_wall(dem_wall& w, WallGeom& geom, double dt
     if (w.type == DEM_WALL_TRIANGLE && !still) triangle_geometry(w, geom);
 }
 
-// With insertion boundaries the walls move before them, in a launch of their own.
-__global__ void __launch_bounds__(128) k_move_walls(DevPtrs d)
+// The walls move in blocks of their own, after the particles' blocks of the
+// kernel that drifts them for the step (w: the thread's index past
+// the particles' blocks). In the launch that opens the step
+// instead they took 3.5 us of every step.
+__device__ __forceinline__ void move_walls(const DevPtrs& d, int w)
 {
-    const int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w < d.n_walls) move_wall(d.walls[w], d.wgeom[w], d.dt);
+    if (w >= 0 && w < d.n_walls) move_wall(d.walls[w], d.wgeom[w], d.dt);
 }
 
 // The skin budget spent since the last rebuild, the last drift included.
@@ -556,6 +557,10 @@ __global__ void __launch_bounds__(256) k_kick_drift(DevPtrs d)
 {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     Control* ctl = d.ctl;
+    if ((int)blockIdx.x >= (d.n + 255) / 256) { // the walls
+        move_walls(d, s - (d.n + 255) / 256 * 256);
+        return;
+    }
     double disp2 = 0.0;
     if (s < d.n) {
         const int c = ctl->cur;

@@ -823,6 +823,10 @@ __global__ void __launch_bounds__(BLOCK, SUM_THREADS_PER_SM / BLOCK) k_sum(DevPt
     const int* uidx = d.uidx[ctl->view.hcur ^ 1]; // of this evaluation
     const bool final_step = (MODE == 0) ? true : (ctl->view.final_step != 0);
     const double dt = d.dt;
+    if ((int)blockIdx.x >= (d.n + BLOCK - 1) / BLOCK) { // the walls, for the next step
+        if (!final_step && !ctl->spare) move_walls(d, s - (d.n + BLOCK - 1) / BLOCK * BLOCK);
+        return;
+    }
     if (s == 0) { // k_units and k_tri are done: the next evaluation starts new lists
         // the springs kept at the pool top in the first time step must not have
         // met this evaluation's items

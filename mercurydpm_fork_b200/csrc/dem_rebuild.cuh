@@ -1,8 +1,7 @@
 // dem_rebuild.cuh -- the neighbour-list rebuild as one cooperative kernel.
 //
 // k_rebuild opens every time step (a cooperative launch: all its blocks are
-// resident together). It moves the walls, and every block decides from the same
-// fields of the control record, which no thread of this launch writes unless it
+// resident together). Every block decides from the same fields of the control record, which no thread of this launch writes unless it
 // rebuilds, whether the skin budget is spent (the Verlet-skin test restating
 // MercuryBase::hGridNeedsRebuilding, MercuryBase.cc:496-535); if not, it returns
 // at once. One thread writes the step's view of the buffers (StepView). A
@@ -121,9 +120,8 @@ __device__ __forceinline__ int block_sum(int v, int* warp_sums)
 }
 
 // step: 1 the launch opens a time step; 0 it only brings the lists up to date
-// (before the initial evaluation). move_walls: they have not moved yet.
-__global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned long long* barrier_ctr, int step,
-                                                         int move_walls)
+// (before the initial evaluation).
+__global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned long long* barrier_ctr, int step)
 {
     Control* ctl = d.ctl;
     const int gt = blockIdx.x * blockDim.x + threadIdx.x, gs = gridDim.x * blockDim.x;
@@ -132,8 +130,6 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
     const int hc = ctl->cur, lo = ctl->lbuf, hh = ctl->hcur ^ flip;
     const double spent = step ? spent_skin(ctl) : 0.0;
     const bool go = ctl->force_rebuild || (step && 2.0 * spent >= ctl->skin);
-    if (move_walls)
-        for (int w = gt; w < d.n_walls; w += gs) move_wall(d.walls[w], d.wgeom[w], d.dt);
     if (gt == 0) {
         StepView& v = ctl->view;
         v.pcur = ctl->pcur ^ flip;

@@ -34,7 +34,7 @@ constexpr int GEMM_BM = 128;
 constexpr int GEMM_BK = 64;
 constexpr int GEMM_THREADS = 256; // 8 warps: warps w and w + 4 share TMEM lanes 32 (w % 4) ..
 constexpr int LAYER_MAX_K = 256;
-constexpr int LAYER_BN = 64;      // output columns of a tile: a batch of 1,024 gives 32 CTAs a layer
+constexpr int LAYER_BN = 32;      // output columns of a tile: a batch of 1,024 gives 64 CTAs a layer
 constexpr unsigned long long WAIT_LIMIT = 1ull << 26; // try_wait polls before giving up
 
 enum Epilogue : int {
@@ -144,6 +144,19 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32])
     for (int i = 0; i < 32; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
+{
+    uint32_t r[16];
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+                 "{%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+                   "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
 // Stage rows [row0, row0 + rows) x k [k0, k0 + 64) of a strided BF16 matrix
 // into the K-major no-swizzle layout: core matrix (row / 8, k / 8) at
 // (row / 8) * 1024 + (k / 8) * 128 bytes, row % 8 selecting its 16-byte row.
@@ -202,11 +215,14 @@ __device__ __forceinline__ void stage_tile_async(unsigned char* dst, const __nv_
 // src[k * s_k + row]; nrows, row0 and s_k multiples of 8, src 16-byte aligned):
 // 8 x 8 blocks, eight 16-byte loads along the rows, transposed in registers.
 // A warp takes 8 K groups x 4 row groups, so a load instruction covers whole
-// 64-byte runs.
-__device__ __forceinline__ void stage_tile_t(unsigned char* dst, const __nv_bfloat16* src, long long s_k, int row0,
-                                             int rows, int nrows, int k0, int K)
+// 64-byte runs. `chunks` consecutive K chunks, `chunk_bytes` apart, at a time.
+__device__ __forceinline__ void stage_tile_t(unsigned char* dst0, const __nv_bfloat16* src, long long s_k, int row0,
+                                             int rows, int nrows, int kfirst, int K, int chunks, int chunk_bytes)
 {
-    for (int it = threadIdx.x; it < rows; it += GEMM_THREADS) { // rows / 8 row groups x 8 K groups
+    for (int t = threadIdx.x; t < rows * chunks; t += GEMM_THREADS) { // rows / 8 row groups x 8 K groups a chunk
+        const int c = t / rows, it = t - c * rows;
+        const int k0 = kfirst + c * GEMM_BK;
+        unsigned char* dst = dst0 + c * chunk_bytes;
         const int g = it & 7, f = it >> 3;
         const int row = row0 + 8 * f;
         uint32_t w[8][4];
@@ -244,7 +260,7 @@ __device__ __forceinline__ void stage_operand(Staging how, unsigned char* dst, c
                                               long long s_k, int row0, int rows, int nrows, int k0, int K)
 {
     if (how == STAGE_ROWS) stage_tile_async(dst, p, s_row, row0, rows, nrows, k0, K);
-    else if (how == STAGE_COLUMNS) stage_tile_t(dst, p, s_k, row0, rows, nrows, k0, K);
+    else if (how == STAGE_COLUMNS) stage_tile_t(dst, p, s_k, row0, rows, nrows, k0, K, 1, 0);
     else stage_tile(dst, p, s_row, s_k, row0, rows, nrows, k0, K);
 }
 
@@ -300,12 +316,13 @@ struct LayerSmem {
 };
 
 // Bound by latency, not throughput (a batch of 1,024 is 0.13 GFLOP a layer):
-// 64-column tiles give 32 CTAs instead of 8, and K is in flight as a whole
-// instead of two chunks. A layer of 1,024 x 256 x 256: 39.7 -> 16.5 us.
+// 32-column tiles give 64 CTAs instead of 8, and K is in flight as a whole
+// instead of two chunks. A layer of 1,024 x 256 x 256: 39.7 -> 9.3 us (16.5 with
+// 64-column tiles and transposed chunks staged one after the other).
 template <int BN>
 __global__ void __launch_bounds__(GEMM_THREADS, 1) k_layer(GemmArgs g)
 {
-    static_assert(BN % 16 == 0 && BN >= 16 && BN <= 64, "UMMA N for M = 128; two warps per lane quarter read 64 columns");
+    static_assert(BN == 16 || BN == 32, "UMMA N for M = 128; two warps per lane quarter read 16 columns each");
     using L = LayerSmem<BN>;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bar;
@@ -319,9 +336,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_layer(GemmArgs g)
     const uint32_t tmem = tile_begin(&bar, 1, &tmem_slot, &failed, tmem_cols(BN));
 
     const Staging how_a = staging_of(g.A, g.a_sm, g.a_sk, g.M), how_b = staging_of(g.B, g.b_sn, g.b_sk, g.N);
+    // transposed operands: every chunk's loads in flight together
+    if (how_a == STAGE_COLUMNS) stage_tile_t(sA, g.A, g.a_sk, m0, GEMM_BM, g.M, 0, g.K, nk, L::A_BYTES);
+    if (how_b == STAGE_COLUMNS) stage_tile_t(sB, g.B, g.b_sk, n0, BN, g.N, 0, g.K, nk, L::B_BYTES);
     for (int c = 0; c < nk; ++c) { // row-contiguous chunks land in order while the later ones are in flight
-        stage_operand(how_a, sA + c * L::A_BYTES, g.A, g.a_sm, g.a_sk, m0, GEMM_BM, g.M, c * GEMM_BK, g.K);
-        stage_operand(how_b, sB + c * L::B_BYTES, g.B, g.b_sn, g.b_sk, n0, BN, g.N, c * GEMM_BK, g.K);
+        if (how_a != STAGE_COLUMNS)
+            stage_operand(how_a, sA + c * L::A_BYTES, g.A, g.a_sm, g.a_sk, m0, GEMM_BM, g.M, c * GEMM_BK, g.K);
+        if (how_b != STAGE_COLUMNS)
+            stage_operand(how_b, sB + c * L::B_BYTES, g.B, g.b_sn, g.b_sk, n0, BN, g.N, c * GEMM_BK, g.K);
         asm volatile("cp.async.commit_group;" ::: "memory");
     }
     for (int c = 0; c < nk; ++c) {
@@ -344,22 +366,22 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_layer(GemmArgs g)
         if (threadIdx.x == 0) atomicExch(g.error, 1u);
     } else {
         // ---- epilogue: thread = accumulator row (tensor-memory lane); the two
-        // warps of a lane quarter take alternate 32-column runs ----
+        // warps of a lane quarter take 16 columns each ----
         const int quarter = warp & 3, cc = warp >> 2;
         const int row = m0 + quarter * 32 + lane;
-        if (cc < (BN + 31) / 32) { // a 16-wide tile reads 32 allocated columns
-            float v[32];
-            tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cc * 32), v);
+        if (16 * cc < BN) {
+            float v[16];
+            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cc * 16), v);
             const long long base = (long long)row * g.ldc;
-            const int nb0 = n0 + cc * 32;
+            const int nb0 = n0 + cc * 16;
             if (row >= g.M) {
-            } else if (cc * 32 + 32 <= BN && nb0 + 32 <= g.N && (g.ldc & 7) == 0) {
-                // a whole 32-column run of this row: 16-byte stores (the row's
-                // 64 or 128 bytes are contiguous)
+            } else if (nb0 + 16 <= g.N && (g.ldc & 7) == 0) {
+                // a whole 16-column run of this row: 16-byte stores (the row's
+                // 32 or 64 bytes are contiguous)
                 const float4* x4 = reinterpret_cast<const float4*>(g.epilogue == EPI_DGELU_BF16 ? g.aux_f32 + base + nb0
                                                                                                  : g.bias + nb0);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
+                for (int i = 0; i < 4; ++i) {
                     const float4 x = x4[i];
                     if (g.epilogue == EPI_DGELU_BF16) {
                         v[4 * i] *= gelu_grad_f(x.x);
@@ -376,13 +398,13 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_layer(GemmArgs g)
                 if (g.epilogue != EPI_DGELU_BF16) {
                     float4* o4 = reinterpret_cast<float4*>(g.out_f32 + base + nb0);
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) o4[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    for (int i = 0; i < 4; ++i) o4[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
                 }
                 if (g.epilogue != EPI_BIAS_F32) {
                     const bool act = g.epilogue != EPI_DGELU_BF16;
                     uint4* o4 = reinterpret_cast<uint4*>(g.out_bf16 + base + nb0);
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
+                    for (int i = 0; i < 2; ++i) {
                         uint32_t w[4];
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
@@ -396,9 +418,9 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1) k_layer(GemmArgs g)
                 }
             } else {
 #pragma unroll
-                for (int i = 0; i < 32; ++i) {
+                for (int i = 0; i < 16; ++i) {
                     const int n = nb0 + i;
-                    if (cc * 32 + i >= BN || n >= g.N) break;
+                    if (n >= g.N) break;
                     const float a = v[i];
                     switch (g.epilogue) {
                     case EPI_BIAS_F32: g.out_f32[base + n] = a + g.bias[n]; break;

@@ -105,13 +105,10 @@ class Surrogate:
 
     def predict(self, x) -> np.ndarray:
         x = _f32(x, (-1, NI))
-        out = np.zeros((len(x), NO), np.float32)
-        for a in range(0, len(x), self.capacity):
+        out = np.empty((len(x), NO), np.float32)
+        for a in range(0, len(x), self.capacity):  # row ranges of contiguous arrays: read and written in place
             b = min(len(x), a + self.capacity)
-            xs = np.ascontiguousarray(x[a:b])
-            ys = np.zeros((b - a, NO), np.float32)
-            self._check(lib().dem_mlp_forward(self._h, _p(xs), b - a, _p(ys)))
-            out[a:b] = ys
+            self._check(lib().dem_mlp_forward(self._h, _p(x[a:b]), b - a, _p(out[a:b])))
         return out
 
     def time_forward(self, n: int, reps: int = 20) -> float:

@@ -89,10 +89,11 @@ struct InstanceDev {
     int n_del;
     uint32_t tri_mask;     // walls (bit w = wall_begin + w) that are triangle walls
     // walls (same bits) whose distance field stays put while the simulation
-    // runs: no translation, and no rotation or one about the wall's own
-    // normal / symmetry axis (infinite and axisymmetric walls). The list
-    // rebuild records which of them are within reach + skin of a particle
-    // (wcand); the others have no unit until the next rebuild
+    // runs (no translation, and no rotation or one about the wall's own
+    // normal / symmetry axis: infinite and axisymmetric walls) or only
+    // translates slowly: at most DevPtrs::wall_step a step, which the rebuild
+    // decision adds up. The list rebuild records which of them are within reach
+    // + skin of a particle (wcand); the others have no unit until the next rebuild
     uint32_t wall_still_mask;
     // walls (same bits) taken out during the run (WallHandler::removeObject):
     // no contacts with them from the next time step on
@@ -130,7 +131,8 @@ struct StepView {
 
 struct Control {
     StepView view;
-    double next_disp_acc;  // disp_acc once this step is under way
+    double next_disp_acc;  // disp_acc and wall_acc once this step is under way
+    double next_wall_acc;
     int cur;               // state buffer holding the current state
     int lbuf;              // unit-list buffer in use
     int pending_flip;      // the last force evaluation wrote the other spring pool and uidx
@@ -142,6 +144,7 @@ struct Control {
     long long steps_done;  // time steps since the upload
     int hcur;              // uidx (and triangle history) buffer of the last evaluation
     double disp_acc;       // sum of per-step maximum displacements since the last rebuild
+    double wall_acc;       // the same of the slowly translating walls
     double skin;
     unsigned long long step_disp2_bits; // max |dx|^2 this step (bits of a non-negative double)
     unsigned int status;   // OR of (1u << DEM_ERR_*)
@@ -233,6 +236,7 @@ struct DevPtrs {
     int has_tri;           // some wall is a triangle wall (k_tri runs)
     double dt;
     double drag;
+    double wall_step; // largest translation a step of the walls in wall_still_mask
 };
 
 } // namespace dem

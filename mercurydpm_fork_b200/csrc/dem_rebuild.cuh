@@ -129,7 +129,9 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
     const int flip = ctl->pending_flip;
     const int hc = ctl->cur, lo = ctl->lbuf, hh = ctl->hcur ^ flip;
     const double spent = step ? spent_skin(ctl) : 0.0;
-    const bool go = ctl->force_rebuild || (step && 2.0 * spent >= ctl->skin);
+    // particles and slow walls may each use half of the skin
+    const double wall_spent = step ? ctl->wall_acc + d.wall_step : 0.0;
+    const bool go = ctl->force_rebuild || (step && (2.0 * spent >= ctl->skin || 2.0 * wall_spent >= ctl->skin));
     if (gt == 0) {
         StepView& v = ctl->view;
         v.pcur = ctl->pcur ^ flip;
@@ -141,6 +143,7 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
             v.lbuf = lo;
             v.hcur = hh;
             ctl->next_disp_acc = spent;
+            ctl->next_wall_acc = wall_spent;
         }
     }
     if (!go) return;
@@ -273,6 +276,7 @@ __global__ void __launch_bounds__(RB_BLOCK, 3) k_rebuild(DevPtrs d, unsigned lon
         ctl->pending_flip = 0;
         ctl->n_units = min(ctl->n_units_next, d.unit_cap);
         ctl->disp_acc = ctl->next_disp_acc = 0.0;
+        ctl->wall_acc = ctl->next_wall_acc = 0.0;
         ctl->force_rebuild = 0;
         ctl->n_rebuilds += 1;
     }

@@ -61,3 +61,24 @@ def test_chunk_size_changes_nothing(gpu, case):
     for other in runs[1:]:
         for k in ("position", "velocity", "angular_velocity", "springs"):
             np.testing.assert_array_equal(other[k], runs[0][k], err_msg=k)
+
+
+@pytest.mark.parametrize("share", [0.024, 0.2])
+def test_wall_that_translates_into_the_bed(gpu, share):
+    """A lid that starts out of reach of every sphere's list and comes down by
+    `share` of the skin a step: below a fortieth it is tested near it alone, its
+    travel brings the list up to date; above, with every sphere."""
+    sc = scenarios.settling_box(n=216, seed=3, box=(6 * 0.999, 6 * 0.999, 6 * 0.999), spacing=0.999 * (1 - 1e-9),
+                                jitter=0.0, vstd=0.0)
+    r = float(sc.radius[0])
+    skin, gap = 0.4 * r, 0.7 * r
+    lid = sc.walls[5]
+    lid.position[2] += gap
+    lid.velocity[2] = -share * skin / sc.time_step
+    steps = int(1.1 * gap / (share * skin))
+    g, o = H.run_gpu(sc, steps), H.run_oracle(sc, steps)
+    assert ((o["contacts"]["is_wall"] == 1) & (o["contacts"]["id_i"] == 5)).sum() > 0
+    assert H.pair_set(g["contacts"]) == H.pair_set(o["contacts"])
+    assert H.rel_err(g["position"], o["position"], 1e-3) < 1e-13
+    for k in ("velocity", "force"):
+        assert H.rel_err(g[k], o[k]) < 1e-9, k

@@ -403,30 +403,58 @@ __device__ __forceinline__ void build_one(const DevPtrs& d, int s, int nb, int& 
     // skin, the other ones always. Triangle walls that stand still: the test
     // of k_units (bounding box, face plane) with the reach widened by the skin,
     // which leaves more than the skin / 2 a particle moves between rebuilds.
+    // A drift may carry a particle near a periodic boundary to the other side
+    // before then, and walls do not repeat with the period: those near the
+    // image it would become count too. Where one image does not cover it
+    // (outside the period, or a period of two skins), all walls do.
     unsigned int wc = 0u, tris = 0u;
     if (!fixed_s) {
         const int nwl = I.wall_end - I.wall_begin;
         const double skin = d.ctl->skin;
+        unsigned int seams = 0u; // directions whose boundary is within the skin
+        V3 shift = zero3();
+        bool all = false;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            if (!((pm >> k) & 1u)) continue;
+            const double lo = (&xs.x)[k] - I.per_lo[k], hi = I.per_hi[k] - (&xs.x)[k];
+            if (lo < skin || hi < skin) {
+                seams |= 1u << k;
+                (&shift.x)[k] = lo < skin ? I.per_L[k] : -I.per_L[k];
+            }
+            all = all || !(fmin(lo, hi) >= -skin) || !(fmax(lo, hi) >= skin);
+        }
         for (int w = 0; w < nwl; ++w) {
             const unsigned int bit = 1u << w;
             if (I.wall_off_mask & bit) continue;
             const int wg = I.wall_begin + w;
-            if (I.tri_mask & bit) {
-                const WallGeom& tg = d.wgeom[wg];
-                const double R = (ps.w + I.max_interaction_distance + skin) * (1.0 + 1e-12);
-                if (!I.tri_static || (triangle_near(tg, xs, R) && triangle_plane_near(tg, xs, R))) tris |= bit;
-                continue;
+            const bool tri = (I.tri_mask & bit) != 0u;
+            bool near = all || !(tri ? I.tri_static : (I.wall_still_mask & bit) != 0u);
+#pragma unroll 1
+            for (unsigned int m = 0u; !near && m < 8u; ++m) { // its own position, then the images
+                if (m & ~seams) continue;
+                const V3 x = v3(xs.x + ((m & 1u) ? shift.x : 0.0), xs.y + ((m & 2u) ? shift.y : 0.0),
+                                xs.z + ((m & 4u) ? shift.z : 0.0));
+                if (tri) {
+                    const WallGeom& tg = d.wgeom[wg];
+                    const double R = (ps.w + I.max_interaction_distance + skin) * (1.0 + 1e-12);
+                    near = triangle_near(tg, x, R) && triangle_plane_near(tg, x, R);
+                } else {
+                    const dem_wall& wall = d.walls[wg];
+                    const double R = ps.w + d.species[I.species_offset + is.y * I.n_species + wall.species].interaction_distance +
+                                     skin;
+                    double dist;
+                    V3 nrm;
+                    near = wall_distance(wall, d.wgeom + wg, x, R, dist, nrm);
+                }
             }
-            if ((I.wall_still_mask >> w) & 1u) {
-                const dem_wall& wall = d.walls[wg];
-                const double R = ps.w + d.species[I.species_offset + is.y * I.n_species + wall.species].interaction_distance +
-                                 skin;
-                double dist;
-                V3 nrm;
-                if (!wall_distance(wall, d.wgeom + wg, xs, R, dist, nrm)) continue;
+            if (!near) continue;
+            if (tri) {
+                tris |= bit;
+            } else {
+                wc |= bit;
+                ++walls;
             }
-            wc |= bit;
-            ++walls;
         }
     }
     if (tris) ++walls;

@@ -990,7 +990,7 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
     // every 9 steps and costs 7 % more per step; the evaluation grows only 3 %)
     if (!(skin > 0.0)) skin = (n > 0) ? 0.4 * rmin_all : 1e-3;
     h->inst.assign(ninst, InstanceDev{});
-    double wall_step = 0.0;
+    double wall_path = 0.0; // the longest way a step that a moving wall makes within its domain
     // levels of all particles; one instance fills the handle's buffer, which
     // keeps its size between uploads (no allocation or zeroing per upload)
     std::vector<int> level_multi(fast ? 0 : n, 0);
@@ -1021,31 +1021,20 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
         I.wall_end = wend[in];
         I.tri_mask = 0u;
         I.tri_static = 1;
-        I.wall_still_mask = 0u;
         I.wall_off_mask = 0u;
         for (int w = wbegin[in]; w < wend[in]; ++w)
             if (h->wall_removed[w]) I.wall_off_mask |= 1u << (w - wbegin[in]);
         for (int w = wbegin[in]; w < wend[in]; ++w) {
             const dem_wall& x = h->walls[w];
             if (x.type == DEM_WALL_TRIANGLE) continue;
-            // A wall that only translates, by less than a fortieth of the skin a step
-            // (20 steps and more use up its half), is tested near it alone, like one
-            // that stands: box of 100,000 in six such walls 70 -> 51 us a step (a unit
-            // for every particle and moving wall otherwise).
-            const double travel = std::sqrt(len2(row3(x.velocity))) * h->cfg.time_step * (1.0 + 1e-9);
-            bool still = travel <= 0.025 * skin;
-            const V3 om = v3(x.angular_velocity[0], x.angular_velocity[1], x.angular_velocity[2]);
-            if (still && len2(om) != 0.0) {
-                // a turn about the normal (infinite) or the axis (axisymmetric)
-                // through the wall's position maps the wall onto itself
-                const V3 ax = quat_axis(Q4{x.orientation[0], x.orientation[1], x.orientation[2], x.orientation[3]});
-                still = (x.type == DEM_WALL_INFINITE || x.type == DEM_WALL_AXISYMMETRIC) &&
-                        len2(cross(om, ax)) <= 1e-24 * len2(om) * len2(ax);
+            set_wall_motion(x, h->cfg.time_step, h->wgeom[w]);
+            double rho2 = 0.0; // its position to the farthest corner
+            for (int k = 0; k < 3; ++k) {
+                const double top = ((D.periodic_mask >> k) & 1u) ? D.periodic_max[k] : D.domain_max[k];
+                const double e = std::max(std::fabs(x.position[k] - I.origin[k]), std::fabs(x.position[k] - top));
+                rho2 += e * e;
             }
-            if (still) {
-                I.wall_still_mask |= 1u << (w - wbegin[in]);
-                wall_step = std::max(wall_step, travel);
-            }
+            wall_path = std::max(wall_path, h->wgeom[w].travel + h->wgeom[w].turn * std::sqrt(rho2));
         }
         for (int k = 0; k < 3; ++k) {
             I.tri_lo[k] = DBL_MAX;
@@ -1137,7 +1126,17 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
     d.any_periodic = 0;
     for (const auto& in : h->inst_desc) d.any_periodic = d.any_periodic || (in.periodic_mask & 7u);
     d.unit_cap = (int)unit_cap;
-    d.wall_step = wall_step;
+    // The steps a list holds for: a slow wall's until it has moved half a skin; at
+    // least 64, because a shorter interval makes the lists anew more often and a
+    // longer one files a fast wall with more spheres (box of 100,000 in six walls
+    // that move by 0.2 skin: 55.4 us a step with 64, 57.4 with 128), and 256 for
+    // small systems, where a rebuild is worth several steps and a unit for every
+    // sphere is cheap (box of 1,000 in such walls: 21.0 us with 64, 19.5 with 256).
+    // Against a unit for every sphere and such wall: 1,000 spheres 19.4 -> 19.5 us,
+    // 10,000 21.3 -> 19.9, 100,000 70.2 -> 54.5; turning off their axis at 100,000
+    // 68.8 -> 53.0; drum of 100,000 with four blades 306 -> 280.
+    const double wall_steps_min = n < 20000 ? 256.0 : 64.0;
+    d.wall_steps = wall_path == 0.0 ? INT_MAX : (int)std::max(wall_steps_min, std::min(1e6, 0.5 * skin / wall_path));
     d.has_tri = 0;
     for (const auto& w : h->walls) d.has_tri = d.has_tri || w.type == DEM_WALL_TRIANGLE;
     d.dt = h->cfg.time_step;
@@ -1151,7 +1150,7 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
                           d.rotation == kept.rotation && d.single_instance == kept.single_instance &&
                           d.n_species_table == kept.n_species_table && d.zero_idist == kept.zero_idist &&
                           d.dt == kept.dt && d.drag == kept.drag && d.has_tri == kept.has_tri &&
-                          d.any_periodic == kept.any_periodic && d.wall_step == kept.wall_step;
+                          d.any_periodic == kept.any_periodic && d.wall_steps == kept.wall_steps;
         if (!same) free_graphs(h);
         for (int b = 0; b < 2; ++b) {
             d.pr[b] = kept.pr[b]; d.vm[b] = kept.vm[b]; d.wi[b] = kept.wi[b]; d.qo[b] = kept.qo[b];

@@ -88,13 +88,6 @@ struct InstanceDev {
     // DeletionBoundary planes: a particle is deleted when del_d - x . del_n < 0
     int n_del;
     uint32_t tri_mask;     // walls (bit w = wall_begin + w) that are triangle walls
-    // walls (same bits) whose distance field stays put while the simulation
-    // runs (no translation, and no rotation or one about the wall's own
-    // normal / symmetry axis: infinite and axisymmetric walls) or only
-    // translates slowly: at most DevPtrs::wall_step a step, which the rebuild
-    // decision adds up. The list rebuild records which of them are within reach
-    // + skin of a particle (wcand); the others have no unit until the next rebuild
-    uint32_t wall_still_mask;
     // walls (same bits) taken out during the run (WallHandler::removeObject):
     // no contacts with them from the next time step on
     uint32_t wall_off_mask;
@@ -131,8 +124,9 @@ struct StepView {
 
 struct Control {
     StepView view;
-    double next_disp_acc;  // disp_acc and wall_acc once this step is under way
-    double next_wall_acc;
+    double next_disp_acc;  // disp_acc and list_age once this step is under way
+    int next_list_age;
+    int pad0;
     int cur;               // state buffer holding the current state
     int lbuf;              // unit-list buffer in use
     int pending_flip;      // the last force evaluation wrote the other spring pool and uidx
@@ -144,7 +138,8 @@ struct Control {
     long long steps_done;  // time steps since the upload
     int hcur;              // uidx (and triangle history) buffer of the last evaluation
     double disp_acc;       // sum of per-step maximum displacements since the last rebuild
-    double wall_acc;       // the same of the slowly translating walls
+    int list_age;          // time steps (moves of the walls) since the last rebuild
+    int pad1;
     double skin;
     unsigned long long step_disp2_bits; // max |dx|^2 this step (bits of a non-negative double)
     unsigned int status;   // OR of (1u << DEM_ERR_*)
@@ -185,10 +180,9 @@ struct DevPtrs {
     // ownership bits: bit k%32 of word own[(k/32)*ncap + i] is set when
     // particle i has the lower id of its entry k's pair
     unsigned int *own;
-    // walls (bit w = wall_begin + w) particle i has units for: still walls
-    // within reach + skin (particles move less than skin / 2 between
-    // rebuilds, so the others cannot be touched), moving walls, and the
-    // triangle walls its one triangle unit tests
+    // walls (bit w = wall_begin + w) particle i has units for: those it can
+    // touch before the next rebuild (build_one), and the triangle walls its one
+    // triangle unit tests
     unsigned int *wcand;
     int2 *unit[2];
     int *uidx[2];
@@ -236,7 +230,9 @@ struct DevPtrs {
     int has_tri;           // some wall is a triangle wall (k_tri runs)
     double dt;
     double drag;
-    double wall_step; // largest translation a step of the walls in wall_still_mask
+    // time steps a list holds for the walls other than triangles that move (but
+    // about their own axis); INT_MAX if none does
+    int wall_steps;
 };
 
 } // namespace dem

@@ -272,7 +272,9 @@ __device__ __forceinline__ bool triangle_plane_near(const WallGeom& tg, V3 x, do
 // take the FP64 test. Contacts themselves are always decided in FP64
 // by the force evaluation, so the superset changes no result. The next row's
 // slot ranges are read ahead and candidates are read BUILD_BATCH at a time.
-// Also the walls of the particle's units (wcand). `pairs` gets the entries the
+// Also the walls of the particle's units (wcand): a wall that moves is filed with
+// the particles it can reach in DevPtrs::wall_steps time steps, after which the
+// lists are made anew in any case. `pairs` gets the entries the
 // particle owns (one unit each), `walls` its wall units.
 constexpr int BUILD_BATCH = 2;
 __device__ __forceinline__ void build_one(const DevPtrs& d, int s, int nb, int& pairs, int& walls)
@@ -399,10 +401,12 @@ __device__ __forceinline__ void build_one(const DevPtrs& d, int s, int nb, int& 
     if (count & 31) d.own[(size_t)(count >> 5) * d.ncap + s] = ownw; // the last, partial word
     d.cnt[s] = count;
 
-    // the walls to test until the next rebuild: still walls within reach +
-    // skin, the other ones always. Triangle walls that stand still: the test
-    // of k_units (bounding box, face plane) with the reach widened by the skin,
-    // which leaves more than the skin / 2 a particle moves between rebuilds.
+    // the walls to test until the next rebuild: those within reach + skin (a
+    // particle moves less than skin / 2 before it) + the wall's own path. A point
+    // at distance rho from the position of a wall sees it come nearer by at most
+    // travel + turn x rho a step, and rho grows by what the two move. Triangle
+    // walls: the test of k_units (bounding box, face plane) with reach + skin; all
+    // of them if any moves.
     // A drift may carry a particle near a periodic boundary to the other side
     // before then, and walls do not repeat with the period: those near the
     // image it would become count too. Where one image does not cover it
@@ -429,7 +433,7 @@ __device__ __forceinline__ void build_one(const DevPtrs& d, int s, int nb, int& 
             if (I.wall_off_mask & bit) continue;
             const int wg = I.wall_begin + w;
             const bool tri = (I.tri_mask & bit) != 0u;
-            bool near = all || !(tri ? I.tri_static : (I.wall_still_mask & bit) != 0u);
+            bool near = all || (tri && !I.tri_static);
 #pragma unroll 1
             for (unsigned int m = 0u; !near && m < 8u; ++m) { // its own position, then the images
                 if (m & ~seams) continue;
@@ -441,11 +445,13 @@ __device__ __forceinline__ void build_one(const DevPtrs& d, int s, int nb, int& 
                     near = triangle_near(tg, x, R) && triangle_plane_near(tg, x, R);
                 } else {
                     const dem_wall& wall = d.walls[wg];
-                    const double R = ps.w + d.species[I.species_offset + is.y * I.n_species + wall.species].interaction_distance +
-                                     skin;
-                    double dist;
-                    V3 nrm;
-                    near = wall_distance(wall, d.wgeom + wg, x, R, dist, nrm);
+                    const WallGeom& geom = d.wgeom[wg];
+                    const double path = d.wall_steps * geom.travel;
+                    const double rho = sqrt(len2(x - row3(wall.position))) + skin + path;
+                    const double R = ps.w +
+                                     d.species[I.species_offset + is.y * I.n_species + wall.species].interaction_distance +
+                                     skin + (path + d.wall_steps * geom.turn * rho);
+                    near = wall_within(wall, &geom, x, R);
                 }
             }
             if (!near) continue;

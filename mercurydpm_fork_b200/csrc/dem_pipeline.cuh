@@ -365,7 +365,7 @@ __global__ void __launch_bounds__(UNIT_BLOCK, MINB) k_units(const __grid_constan
         ctl->force_rebuild = 0;
         if (MODE == 1) {
             ctl->disp_acc = ctl->next_disp_acc;
-            ctl->wall_acc = ctl->next_wall_acc;
+            ctl->list_age = ctl->next_list_age;
             ctl->step_disp2_bits = 0ull;
             ctl->steps_left -= 1;
             ctl->steps_done += 1;

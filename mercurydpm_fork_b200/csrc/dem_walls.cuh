@@ -42,6 +42,9 @@ struct WallGeom {
     double tel[3];                    // edge lengths (edgeLength_)
     double tfn[3];                    // unit face normal (faceNormal_)
     double tlo[3], thi[3];            // bounding box of the vertices (vertexMin_, vertexMax_)
+    // per time step: the wall's translation, and the angle it turns by about its
+    // position (0 where that maps the wall onto itself)
+    double travel, turn;
 };
 
 __host__ __device__ __forceinline__ Q4 wall_q(const dem_wall& w)
@@ -313,7 +316,43 @@ __host__ __device__ __forceinline__ bool wall_distance(const dem_wall& w, const 
     return true;
 }
 
+// Whether x may be within R of a wall other than a triangle: the test that opens
+// wall_distance (every face nearer than R). Each face distance changes by at
+// most the distance x moves, so a point near enough for wall_distance passes
+// here with R widened by its path; the edge and corner branches of
+// intersection_distance, which pick their line or corner by R, give no such bound.
+__host__ __device__ __forceinline__ bool wall_within(const dem_wall& w, const WallGeom* geom, V3 x, double R)
+{
+    const Q4 q = wall_q(w);
+    const V3 wp = v3(w.position[0], w.position[1], w.position[2]);
+    if (w.type == DEM_WALL_INFINITE) return !(quat_plane_distance(q, x, wp) >= R);
+    V3 local;
+    if (w.type == DEM_WALL_AXISYMMETRIC) {
+        const V3 po = x - wp;
+        const V3 axis = quat_axis(q);
+        const double a = dot(po, axis);
+        local = v3(sqrt(len2(po - a * axis)), 0.0, a);
+    } else {
+        local = quat_to_body(q, x - wp);
+    }
+    for (unsigned k = 0; k < (unsigned)w.n_faces; ++k)
+        if (face_distance(*geom, k, local) >= R) return false;
+    return w.n_faces > 0;
+}
+
 // ---- host-side set-up --------------------------------------------------
+
+// The per-step motion of a wall other than a triangle (WallGeom::travel, turn).
+__host__ inline void set_wall_motion(const dem_wall& w, double dt, WallGeom& g)
+{
+    const V3 om = row3(w.angular_velocity), axis = quat_axis(wall_q(w));
+    // a turn about the normal (infinite) or the axis (axisymmetric) through the
+    // wall's position maps the wall onto itself
+    const bool own = (w.type == DEM_WALL_INFINITE || w.type == DEM_WALL_AXISYMMETRIC) &&
+                     len2(cross(om, axis)) <= 1e-24 * len2(om) * len2(axis);
+    g.travel = sqrt(len2(row3(w.velocity))) * dt * (1.0 + 1e-9);
+    g.turn = own ? 0.0 : sqrt(len2(om)) * dt * (1.0 + 1e-9);
+}
 
 // Quaternion::setOrientationViaNormal (Quaternion.cc:543-567), which first
 // normalises the normal: the rotation taking (1, 0, 0) to the normal.

@@ -66,8 +66,7 @@ def test_chunk_size_changes_nothing(gpu, case):
 @pytest.mark.parametrize("share", [0.024, 0.2])
 def test_wall_that_translates_into_the_bed(gpu, share):
     """A lid that starts out of reach of every sphere's list and comes down by
-    `share` of the skin a step: below a fortieth it is tested near it alone, its
-    travel brings the list up to date; above, with every sphere."""
+    `share` of the skin a step: its list holds for the steps it is made for."""
     sc = scenarios.settling_box(n=216, seed=3, box=(6 * 0.999, 6 * 0.999, 6 * 0.999), spacing=0.999 * (1 - 1e-9),
                                 jitter=0.0, vstd=0.0)
     r = float(sc.radius[0])

@@ -52,11 +52,15 @@ int  dem_mlp_forward(dem_mlp *h, const float *x, int n, float *y);
 /* Loss and gradient (DEM_MLP_NPARAMS floats) of the batch, no update. */
 int  dem_mlp_gradients(dem_mlp *h, const float *x, const float *t, int n, float *loss, float *grads);
 /* One Adam step (beta1 0.9, beta2 0.999, eps 1e-8) on the batch; *loss is the
- * batch loss before the update. */
+ * batch loss before the update. A step that ends in DEM_MLP_ERR_TIMEOUT leaves
+ * parameters, moments and the step count as they were. */
 int  dem_mlp_train_step(dem_mlp *h, const float *x, const float *t, int n, float lr, float *loss);
 /* Device time of the forward pass (inputs already on the device from the
  * last call) for n rows, averaged over reps launches: *ms per pass. */
 int  dem_mlp_time_forward(dem_mlp *h, int n, int reps, float *ms);
+/* Sets the device status that a kernel sets when one of its waits runs out: the
+ * next call finds it, returns DEM_MLP_ERR_TIMEOUT and clears it. */
+int  dem_mlp_selftest_expire(dem_mlp *h);
 const char *dem_mlp_last_error(dem_mlp *h);
 void dem_mlp_destroy(dem_mlp *h);
 

@@ -132,13 +132,15 @@ __global__ void k_to_bf16(const float* p, long long n, __nv_bfloat16* out)
 
 // The gradient of parameter i from the slices' partial sums in slice order, the
 // loss from the blocks' parts, and (step) Adam (Kingma and Ba 2015) with bias
-// correction, which refreshes the BF16 copy.
+// correction, which refreshes the BF16 copy. Where a wait of this pass ran out
+// (*error), a slice's sums are not of this batch: nothing changes.
 __global__ void __launch_bounds__(256) k_reduce_params(const float* partial, int slices, long long stride, const float* loss_part,
                                                        int loss_blocks, float loss_scale, float* loss, float* g, bool step,
                                                        float* p, float* m, float* v, float lr, float bc1, float bc2,
-                                                       __nv_bfloat16* wb)
+                                                       __nv_bfloat16* wb, const unsigned* error)
 {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (*error) return;
     if (i == 0) {
         float s = 0.f;
         for (int b = 0; b < loss_blocks; ++b) s += loss_part[b];
@@ -280,7 +282,7 @@ int backward(Mlp* h, int n, float lr = 0.f, float bc1 = 1.f, float bc2 = 1.f)
     k_weight_grads<<<dim3(tiles, slices), GEMM_THREADS, smem, h->stream>>>(a);
     k_reduce_params<<<grid1(NPARAM, 256), 256, 0, h->stream>>>(h->partial, slices, PARAM_STRIDE, h->loss_part, loss_blocks,
                                                                3.0f * (float)n, h->loss, h->g, lr > 0.f, h->p, h->m, h->v,
-                                                               lr, bc1, bc2, h->wb);
+                                                               lr, bc1, bc2, h->wb, h->d_error);
     CK(cudaGetLastError());
     return DEM_MLP_OK;
 }
@@ -450,9 +452,10 @@ int dem_mlp_train_step(dem_mlp* h, const float* x, const float* t, int n, float 
     const float bc1 = 1.0f - std::pow(0.9f, (float)(h->step + 1));
     const float bc2 = 1.0f - std::pow(0.999f, (float)(h->step + 1));
     if ((rc = load_batch(h, x, t, n)) || (rc = forward(h, n)) || (rc = backward(h, n, lr, bc1, bc2))) return rc;
-    h->step += 1;
     if (loss) CK(cudaMemcpyAsync(loss, h->loss, sizeof(float), cudaMemcpyDeviceToHost, h->stream));
-    return check_device_status(h);
+    if ((rc = check_device_status(h))) return rc;
+    h->step += 1;
+    return DEM_MLP_OK;
 }
 
 int dem_mlp_time_forward(dem_mlp* h, int n, int reps, float* ms)
@@ -474,6 +477,15 @@ int dem_mlp_time_forward(dem_mlp* h, int n, int reps, float* ms)
     if (rc) return rc;
     *ms = t / reps;
     return check_device_status(h);
+}
+
+int dem_mlp_selftest_expire(dem_mlp* h)
+{
+    if (!h) return DEM_MLP_ERR_BAD_INPUT;
+    CK(cudaSetDevice(h->device));
+    CK(cudaMemsetAsync(h->d_error, 1, sizeof(unsigned), h->stream));
+    CK(cudaStreamSynchronize(h->stream));
+    return DEM_MLP_OK;
 }
 
 const char* dem_mlp_last_error(dem_mlp* h) { return h ? h->err.c_str() : "null handle"; }

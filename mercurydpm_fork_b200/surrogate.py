@@ -35,6 +35,7 @@ def lib() -> C.CDLL:
             "dem_mlp_gradients": (C.c_int, [C.c_void_p, _pf, _pf, C.c_int, _pf, _pf]),
             "dem_mlp_train_step": (C.c_int, [C.c_void_p, _pf, _pf, C.c_int, C.c_float, _pf]),
             "dem_mlp_time_forward": (C.c_int, [C.c_void_p, C.c_int, C.c_int, _pf]),
+            "dem_mlp_selftest_expire": (C.c_int, [C.c_void_p]),
             "dem_mlp_last_error": (C.c_char_p, [C.c_void_p]),
             "dem_mlp_destroy": (None, [C.c_void_p]),
         }

@@ -38,3 +38,25 @@ def test_gradients_at_the_edges_of_tiles_and_slices(gpu, n):
     # first Adam step from rest: m / bc1 = g, v / bc2 = g^2 (FP32 evaluation: 1e-6 of a step of 1e-3, and p's rounding)
     g = g.astype(np.float64)
     np.testing.assert_allclose(p1, p0 - 1e-3 * g / (np.abs(g) + 1e-8), rtol=1e-6, atol=2e-8 + 1e-3 * 1e-4)
+
+
+def test_a_step_whose_wait_ran_out_changes_nothing(gpu):
+    """A kernel whose wait runs out leaves its result unwritten, so the sums over
+    the slices of such a pass hold older values: the step reports it and touches
+    neither parameters, moments nor the step count. (The status is set from the
+    host; no wait is made to run out.)"""
+    from mercurydpm_fork_b200.surrogate import SurrogateError, lib
+    s, twin = _net(), _net()
+    batches = [_data(n, seed=n) for n in (300, 1024, 128)]
+    for net in (s, twin):
+        net.train_step(*batches[0])
+    before = s.params()
+    assert lib().dem_mlp_selftest_expire(s._h) == 0
+    with pytest.raises(SurrogateError, match="2: "):
+        s.train_step(*batches[1])
+    np.testing.assert_array_equal(s.params(), before)
+    for b in batches[1:]:
+        assert s.train_step(*b) == twin.train_step(*b)
+        np.testing.assert_array_equal(s.params(), twin.params())
+    s.close()
+    twin.close()

@@ -57,29 +57,7 @@ struct GemmArgs {
     unsigned int* error;     // set to 1 when a wait runs out
 };
 
-// z Phi(z) = max(z, 0) - a Phi(-a), a = |z|, with Phi(-a) = exp(-a^2 / 2) R(a) and
-// R (half the scaled complementary error function of a / sqrt 2) a polynomial of
-// degree 6 in 1 / (1 + 0.27 a): least squares at Chebyshev nodes of that variable
-// over a <= 9, 1e-8 of the result; beyond, the exponential is below FP32's
-// rounding. In FP32 over |z| <= 9 the largest error is 2.4e-7 (0.5 z (1 + erff):
-// 4.4e-7, all of the negative tail's digits), at half the instructions and
-// without a branch: the inference kernel, bound by them, 122 -> 104 us for 65,536
-// rows. Infinity and NaN go through the first term as before.
-__device__ __forceinline__ float gelu_f(float z)
-{
-    const float a = fminf(fabsf(z), 20.0f);
-    float t, e;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t) : "f"(fmaf(0.27f, a, 1.0f)));
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(a * a * -0.72134752f)); // -log2(e) / 2
-    float q = -0.133035123f;
-    q = fmaf(q, t, 0.565792561f);
-    q = fmaf(q, t, -0.535542428f);
-    q = fmaf(q, t, 0.51941371f);
-    q = fmaf(q, t, -0.0556198321f);
-    q = fmaf(q, t, 0.141979784f);
-    q = fmaf(q, t, -0.00298865652f);
-    return fmaf(0.5f, z, 0.5f * fabsf(z)) - q * e * a;
-}
+__device__ __forceinline__ float gelu_f(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
 
 // d/dz of z Phi(z): Phi(z) + z phi(z)
 __device__ __forceinline__ float gelu_grad_f(float z)

@@ -481,8 +481,8 @@ int  dem_last_step_stats(dem_handle *h, double *ms, int64_t *kernel_launches,
                          int64_t *rebuilds);
 int  dem_get_info(dem_handle *h, int64_t *n_particles, int64_t *max_neighbors,
                   int64_t *n_cells);
-/* Device memory held by the handle's particle, list and contact arrays, and
- * the contact capacity (items of one evaluation) they were sized for. */
+/* Device memory held by the handle's particle, list and contact arrays and by
+ * the workspace it keeps between calls (at most 512 MB), and the contact capacity (items of one evaluation) they were sized for. */
 int  dem_get_memory(dem_handle *h, int64_t *device_bytes, int64_t *contact_capacity);
 /* Neighbour-list entries, live particle contacts and wall contacts of the
  * current state (the sizes the per-step byte count is made of). */
@@ -500,6 +500,11 @@ int  dem_time_force_kernel(dem_handle *h, int reps, double *ms_per_launch);
  * reports DEM_ERR_TIMEOUT; *status receives the status word the kernel wrote
  * (1 << DEM_ERR_TIMEOUT expected). The handle stays usable afterwards. */
 int  dem_selftest_wait_expiry(dem_handle *h, int64_t polls, uint32_t *status);
+/* Self-test of calls on a full device (no reference counterpart): from now on
+ * the handle gets no workspace of more than `bytes`, as if the device had no
+ * room for it (UINT64_MAX: no limit). The contact downloads then sort on the
+ * host; dem_reduce and dem_cg_eval report DEM_ERR_CUDA. */
+int  dem_selftest_workspace_limit(dem_handle *h, uint64_t bytes);
 /* Autotuner (the reference's HGridOptimiser, Kernel/HGridOptimiser.cc, picks
  * cell sizes offline from a cost model; the engine's cells follow the
  * reference's HGrid levels, and what is tuned instead are its kernels' launch

@@ -10,6 +10,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "dem_engine.cuh"
@@ -72,6 +73,7 @@ struct Handle {
     double* d_stage = nullptr;         // caller-layout particle staging (18 words per slot)
     char* d_scratch = nullptr;         // workspace kept between calls (Scratch), at most SCRATCH_KEEP bytes
     size_t scratch_bytes = 0;
+    size_t scratch_limit = SIZE_MAX;   // above it no workspace is to be had (dem_selftest_workspace_limit)
     double* d_batch = nullptr;         // per-instance balance rows of dem_reduce_batch
     std::vector<long long> layout;     // sizes the device arrays were allocated for
     Control* d_ctl = nullptr;
@@ -135,7 +137,8 @@ int dalloc(Handle* h, T** p, size_t count)
 // mapped anew each time (measured: 0.45 ms of a dem_reduce of 1,000 particles,
 // about 2 ms of a coarse-graining evaluation of 200,000). Larger needs (some
 // millions of contacts) are taken and given back per call. Calls on a handle are
-// serialised on its stream, so one block serves them all.
+// serialised on its stream, so one block serves them all. It goes with the
+// particle arrays when a simulation of other sizes replaces them.
 constexpr size_t SCRATCH_KEEP = 512ull << 20;
 struct Scratch {
     Handle* h;
@@ -144,7 +147,14 @@ struct Scratch {
     explicit Scratch(Handle* handle) : h(handle) {}
     Scratch(const Scratch&) = delete;
     Scratch& operator=(const Scratch&) = delete;
+    // a failure leaves no error behind for the next launch to find
     cudaError_t take(size_t bytes)
+    {
+        const cudaError_t e = bytes > h->scratch_limit ? cudaErrorMemoryAllocation : allocate(bytes);
+        if (e != cudaSuccess) cudaGetLastError();
+        return e;
+    }
+    cudaError_t allocate(size_t bytes)
     {
         if (bytes > SCRATCH_KEEP) {
             const cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&p), bytes, h->stream);
@@ -193,6 +203,9 @@ void free_particle_arrays(Handle* h)
     free_graphs(h);
     for (void* p : h->allocs) cudaFree(p);
     h->allocs.clear();
+    if (h->d_scratch) cudaFree(h->d_scratch);
+    h->d_scratch = nullptr;
+    h->scratch_bytes = 0;
     h->alloc_bytes = 0;
     h->d_records = nullptr;
     h->record_capacity = 0;
@@ -1677,6 +1690,22 @@ int dem_download_walls(dem_handle* hh, dem_wall* walls, int n)
     return DEM_OK;
 }
 
+// The same on the host, where the device has no room for the sorts and the
+// arrays: these downloads need no device memory.
+static int download_records_host(Handle* h, int64_t m, const RecordArrays& to)
+{
+    std::vector<ContactRecord> rec(h->n_records);
+    CU(cudaMemcpyAsync(rec.data(), h->d_records, rec.size() * sizeof(ContactRecord), cudaMemcpyDeviceToHost, h->stream));
+    CU(cudaStreamSynchronize(h->stream));
+    for (auto& r : rec)
+        if (r.is_wall) r.id_i = h->wall_caller[r.id_i];
+    std::stable_sort(rec.begin(), rec.end(), [](const ContactRecord& a, const ContactRecord& b) {
+        return std::tie(a.is_wall, a.id_p, a.id_i) < std::tie(b.is_wall, b.id_p, b.id_i);
+    });
+    for (int64_t k = 0; k < m; ++k) put_record(to, (size_t)k, rec[k], rec[k].id_i);
+    return DEM_OK;
+}
+
 // The first m contact records of the last evaluation, in the order the contact
 // downloads report them (dem_records.cuh), into the host arrays of `to` (null: not
 // asked for).
@@ -1704,7 +1733,7 @@ static int download_records(Handle* h, int64_t m, const RecordArrays& to)
     for (Out& o : out)
         if (o.host) o.at = a.take(n * o.width);
     Scratch scratch(h);
-    CU(scratch.take(a.total));
+    if (scratch.take(a.total) != cudaSuccess) return download_records_host(h, m, to);
     auto at = [&](size_t off) { return (void*)(scratch.p + off); };
     auto dev = [&](const Out& o) { return o.host ? at(o.at) : nullptr; };
     unsigned *k0 = (unsigned*)at(o_key0), *k1 = (unsigned*)at(o_key1);
@@ -1970,7 +1999,7 @@ int dem_get_memory(dem_handle* hh, int64_t* device_bytes, int64_t* contact_capac
 {
     Handle* h = reinterpret_cast<Handle*>(hh);
     if (!h) return DEM_ERR_BAD_INPUT;
-    if (device_bytes) *device_bytes = (int64_t)h->alloc_bytes;
+    if (device_bytes) *device_bytes = (int64_t)(h->alloc_bytes + h->scratch_bytes);
     if (contact_capacity) *contact_capacity = h->d.item_cap;
     return DEM_OK;
 }
@@ -1983,9 +2012,7 @@ int dem_get_counts(dem_handle* hh, int64_t* list_entries, int64_t* contacts, int
     CU(cudaSetDevice(h->device));
     unsigned long long v[3] = {0, 0, 0};
     const unsigned nr = h->records_valid ? h->n_records : 0;
-    Scratch scratch(h);
-    CU(scratch.take(sizeof(v)));
-    unsigned long long* dv = reinterpret_cast<unsigned long long*>(scratch.p);
+    unsigned long long* dv = reinterpret_cast<unsigned long long*>(h->d_stage); // 32 rows at least
     CU(cudaMemsetAsync(dv, 0, sizeof(v), h->stream));
     const long long most = std::max<long long>(h->d.n, nr);
     k_count<<<(unsigned)std::min<long long>(grid_for(most, 256), 4ll * h->sm_count), 256, 0, h->stream>>>(h->d, nr, dv);
@@ -2180,7 +2207,6 @@ void dem_destroy(dem_handle* hh)
     cudaSetDevice(h->device);
     if (h->stream) cudaStreamSynchronize(h->stream);
     free_particle_arrays(h);
-    if (h->d_scratch) cudaFree(h->d_scratch);
     if (h->d_rtmp) cudaFree(h->d_rtmp);
     if (h->d_rstats) cudaFree(h->d_rstats);
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -2211,6 +2237,14 @@ int dem_batch_run(dem_handle* hh, int nsteps, dem_globals* out)
     int rc = dem_step(hh, nsteps);
     if (rc) return rc;
     return dem_reduce_batch(hh, 0, (int)h->inst.size(), out);
+}
+
+int dem_selftest_workspace_limit(dem_handle* hh, uint64_t bytes)
+{
+    Handle* h = reinterpret_cast<Handle*>(hh);
+    if (!h) return DEM_ERR_BAD_INPUT;
+    h->scratch_limit = (size_t)bytes;
+    return DEM_OK;
 }
 
 int dem_selftest_wait_expiry(dem_handle* hh, int64_t polls, uint32_t* status)

@@ -48,25 +48,30 @@ struct RecordArrays {
     double *contact_point, *normal, *tangential;   // 3 each
 };
 
+__host__ __device__ __forceinline__ void put_record(const RecordArrays& a, size_t k, const ContactRecord& r, int id_i)
+{
+    if (a.id_p) a.id_p[k] = r.id_p;
+    if (a.id_i) a.id_i[k] = id_i;
+    if (a.is_wall) a.is_wall[k] = r.is_wall;
+    if (a.periodic) a.periodic[k] = r.periodic;
+    if (a.overlap) a.overlap[k] = r.overlap;
+    if (a.springs)
+        for (int c = 0; c < 9; ++c) a.springs[9 * k + c] = r.springs[c];
+    for (int c = 0; c < 3; ++c) {
+        if (a.force) a.force[3 * k + c] = r.force[c];
+        if (a.contact_point) a.contact_point[3 * k + c] = r.contact_point[c];
+        if (a.normal) a.normal[3 * k + c] = r.normal[c];
+        if (a.tangential) a.tangential[3 * k + c] = r.tangential[c];
+    }
+}
+
 __global__ void __launch_bounds__(256) k_record_arrays(const ContactRecord* rec, unsigned n, const int* order,
                                                        const int* wall_caller, RecordArrays a)
 {
     const unsigned k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const ContactRecord& r = rec[order[k]];
-    if (a.id_p) a.id_p[k] = r.id_p;
-    if (a.id_i) a.id_i[k] = reported_i(r, wall_caller);
-    if (a.is_wall) a.is_wall[k] = r.is_wall;
-    if (a.periodic) a.periodic[k] = r.periodic;
-    if (a.overlap) a.overlap[k] = r.overlap;
-    if (a.springs)
-        for (int c = 0; c < 9; ++c) a.springs[9 * (size_t)k + c] = r.springs[c];
-    for (int c = 0; c < 3; ++c) {
-        if (a.force) a.force[3 * (size_t)k + c] = r.force[c];
-        if (a.contact_point) a.contact_point[3 * (size_t)k + c] = r.contact_point[c];
-        if (a.normal) a.normal[3 * (size_t)k + c] = r.normal[c];
-        if (a.tangential) a.tangential[3 * (size_t)k + c] = r.tangential[c];
-    }
+    put_record(a, k, r, reported_i(r, wall_caller));
 }
 
 // forces and torques (engine order) -> caller order

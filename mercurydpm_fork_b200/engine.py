@@ -589,7 +589,7 @@ class DemEngine:
                     max_neighbors=cap.value, n_cells=cells.value)
 
     def memory(self) -> dict:
-        """Device bytes held by the handle's arrays and the contact capacity
+        """Device bytes held by the handle's arrays and kept workspace, and the contact capacity
         (items of one evaluation) the spring storage was sized for."""
         b = C.c_int64(0)
         cap = C.c_int64(0)

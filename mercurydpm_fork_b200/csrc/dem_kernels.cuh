@@ -307,7 +307,11 @@ __device__ __forceinline__ void build_one(const DevPtrs& d, int s, int nb, int& 
     bool overflow = false;
     unsigned int ownw = 0u; // ownership bits of the list word being filled
     for (int lvl = 0; lvl < I.n_levels; ++lvl) {
-        const double reach = ps.w + I.level_rmax[lvl] + extra;
+        double reach = ps.w + I.level_rmax[lvl] + extra;
+        // and as far as the FP32 test accepts, so that both particles of a pair
+        // find each other: its margin, with the partner's coordinates (at most
+        // reach and a period from these) and the rounding of all of them
+        reach += 4.0 * U20 * ((double)ms + lmax + 2.0 * reach);
         int lox, hix, loy, hiy, loz, hiz;
         cell_range(I, lvl, 0, xs.x, reach, lox, hix);
         cell_range(I, lvl, 1, xs.y, reach, loy, hiy);

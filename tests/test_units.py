@@ -81,3 +81,21 @@ def test_wall_that_translates_into_the_bed(gpu, share):
     assert H.rel_err(g["position"], o["position"], 1e-3) < 1e-13
     for k in ("velocity", "force"):
         assert H.rel_err(g[k], o[k]) < 1e-9, k
+
+
+@pytest.mark.parametrize("l_d,skin", [(50.0, 0.05), (50.0, 0.0501), (31.0, 0.05)])
+def test_lists_are_symmetric_at_the_edge_of_the_reach(gpu, l_d, skin):
+    """Spheres 1.05 diameters apart with a skin of 0.05: thousands of pairs lie
+    within the FP32 test's margin of the reach, some of them with a cell boundary
+    in between. A list that one partner alone holds is an error of the run."""
+    n = 50_000 if l_d > 40 else 20_000
+    sc = scenarios.triangle_floor(n=n, seed=1, drop_d=0.02, v0=0.5, l_d=l_d)
+    e = sc.engine(skin=skin * 1e-3)
+    e.step(150)
+    x, rebuilds = e.download()["position"], e.stats()["rebuilds"]
+    e.close()
+    assert rebuilds >= 3
+    e = sc.engine()
+    e.step(150)
+    assert H.rel_err(x, e.download()["position"], 1e-3) < 1e-13
+    e.close()

@@ -1049,19 +1049,12 @@ int dem_upload_particles(dem_handle* hh, const dem_particles_soa* p)
             }
             wall_path = std::max(wall_path, h->wgeom[w].travel + h->wgeom[w].turn * std::sqrt(rho2));
         }
-        for (int k = 0; k < 3; ++k) {
-            I.tri_lo[k] = DBL_MAX;
-            I.tri_hi[k] = -DBL_MAX;
-        }
         for (int w = wbegin[in]; w < wend[in]; ++w) {
             const dem_wall& x = h->walls[w];
             if (x.type != DEM_WALL_TRIANGLE) continue;
             I.tri_mask |= 1u << (w - wbegin[in]);
-            for (int k = 0; k < 3; ++k) {
+            for (int k = 0; k < 3; ++k)
                 I.tri_static = I.tri_static && x.velocity[k] == 0.0 && x.angular_velocity[k] == 0.0;
-                I.tri_lo[k] = std::min(I.tri_lo[k], h->wgeom[w].tlo[k]);
-                I.tri_hi[k] = std::max(I.tri_hi[k], h->wgeom[w].thi[k]);
-            }
         }
         fill_deletions(h, I, in);
         std::vector<int> lv_multi;

@@ -91,8 +91,7 @@ struct InstanceDev {
     // walls (same bits) taken out during the run (WallHandler::removeObject):
     // no contacts with them from the next time step on
     uint32_t wall_off_mask;
-    int tri_static;        // every triangle wall of the instance stands still: tri_lo/hi hold
-    double tri_lo[3], tri_hi[3]; // the bounding box of all their vertices
+    int tri_static;        // every triangle wall of the instance stands still
     double del_n[DEM_MAX_DELETION_PER_INSTANCE][3];
     double del_d[DEM_MAX_DELETION_PER_INSTANCE];
 };

@@ -6,10 +6,11 @@
 //               turned into a Verlet-skin test), which every block decides for
 //               itself (dem_rebuild.cuh). A rebuild: cell keys per
 //               HGrid level, counting sort, per-cell ordering by particle id,
-//               permutation gather of the state, neighbour lists with
-//               contact-history carry-over, their reverse index (replaces
-//               HGrid buckets + InteractionHandler lookup, Mercury3D.cc:224-416,
-//               InteractionHandler.cc:103-174). The per-item steps are below.
+//               permutation gather of the state, neighbour lists, the units
+//               made from them, and the contact history carried to those
+//               (replaces HGrid buckets + InteractionHandler lookup,
+//               Mercury3D.cc:224-416, InteractionHandler.cc:103-174). The
+//               per-item steps are below.
 //   force       k_units -> k_sum (dem_pipeline.cuh): the exact FP64 contact
 //               predicate (BaseParticle::getInteractionWith,
 //               BaseParticle.cc:688-710) and the contact law once per contact

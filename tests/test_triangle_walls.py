@@ -101,7 +101,8 @@ def test_moving_triangle_walls_match_reference(gpu):
 @needs_reference
 def test_periodic_triangle_floor_matches_reference(gpu):
     """Grouped triangles spanning a periodic square (x and y), spheres
-    arriving at 1 m/s: contacts near the periodic seams, list rebuilds."""
+    arriving at 1 m/s from above: contacts of all kinds, list rebuilds. (They
+    move too little sideways to cross a seam: test_periodic_walls.)"""
     from mercurydpm_fork_b200 import scenarios
     sc = scenarios.triangle_floor(n=1500, l_d=20.0, amplitude_d=0.3, drop_d=0.05, v0=1.0)
     g = H.run_gpu(sc, 200)
@@ -116,8 +117,9 @@ def test_periodic_triangle_floor_matches_reference(gpu):
 @pytest.mark.gpu
 @needs_reference
 def test_static_mesh_box_margin_matches_reference(gpu):
-    """k_detect skips the triangle tests of a particle outside the bounding
-    box of a static mesh widened by its reach (radius + interaction distance).
+    """A rebuild files a static triangle with the particles in its bounding box
+    widened by their reach (radius + interaction distance + skin), and k_units
+    tests those against the box widened by radius + interaction distance.
     Spheres placed around a 10 x 10 diameter patch at that margin (a hair
     inside and outside it, and exactly on it), others a tenth of a diameter
     out and moving in, others dropping onto the patch's corners: the

@@ -459,16 +459,10 @@ __device__ __forceinline__ void build_one(const DevPtrs& d, int s, int nb, int& 
                     near = wall_within(wall, &geom, x, R);
                 }
             }
-            if (!near) continue;
-            if (tri) {
-                tris |= bit;
-            } else {
-                wc |= bit;
-                ++walls;
-            }
+            if (near) (tri ? tris : wc) |= bit;
         }
     }
-    if (tris) ++walls;
+    walls = __popc(wc) + (tris ? 1 : 0);
     d.wcand[s] = wc | tris;
 }
 

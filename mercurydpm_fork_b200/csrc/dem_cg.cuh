@@ -522,8 +522,11 @@ __device__ __forceinline__ void cg_walk_wide(const int (&p0)[3], const int (&p1)
     }
 }
 
-// Bound by FP64 issue (two error functions and an exponential per contact and
-// point in reach). One warp per point read every candidate's record from L2
+// Bound by the latency of its FP64 chains (two error functions and an exponential
+// per contact and point in reach) in warps that are partly idle: of a box of
+// 20,000 on 20 x 20 x 24 points, 18.8 of 32 lanes active (the others' entries
+// failed the range or cutoff test), 16 warps per SM, 44 % of the issue slots, 27 %
+// of the FP64 pipe, DRAM idle. One warp per point read every candidate's record from L2
 // again for each point, some 6.8 GB per evaluation of the 200,000 chute on 100 x
 // 50 points, and searched the whole period once a contact crossed it. Tiles of
 // 8 points with a list of their own for those contacts: 1.25 -> 0.75 ms there,
